@@ -35,7 +35,7 @@ struct flash_hy_ctx {
   int *d_blk_nbr;             // uniform grids: [nblocks][6] face neighbours
   fhy::TmaLine *tma_run;      // run kernels' maps (2 state buffers x 3 directions), or NULL
   int *d_runs[3];             // per direction: [nblocks / kMxRun][kMxRun + 2]
-  void *d_cflq;               // [nblocks][kMxRun] CFL candidates of the run quarters
+  fhy::CflCand *d_cflq;       // 3D: [nblocks][kCflParts] CFL candidates of the CTAs that share a block
   int list_cap;
   int *h_list;               // 0-based copy of a caller's 1-based block list
   int h_list_cap;
@@ -213,7 +213,7 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t
                                   const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 static_assert(fhy::kMxRun == FLASH_HY_MX_RUN, "the run length of the header and the kernels agree");
-static fhy::TmaLine *make_tma_maps(flash_hy_ctx *c, int K = 1) {
+static fhy::TmaLine *make_tma_maps(flash_hy_ctx *c, int parts = 1) {
   if (c->ndim != 3 || c->nx != 8 || c->ny != 8 || c->nz != 8) return nullptr;
   static EncodeTiledFn encode = nullptr;
   if (!encode) {
@@ -231,9 +231,9 @@ static fhy::TmaLine *make_tma_maps(flash_hy_ctx *c, int K = 1) {
   const cuuint64_t dims[3] = {8, 8, (cuuint64_t)c->nblocks * 8};
   const cuuint64_t strides[2] = {8 * sizeof(double), 64 * sizeof(double)};
   const cuuint32_t one[3] = {1, 1, 1};
-  // runs (K > 1): 1/K of the slower transverse axis (z for the x and y
-  // sweeps, y for the z sweep)
-  const cuuint32_t q = (cuuint32_t)(8 / K);
+  // runs (parts > 1): 1/parts of the slower transverse axis (z for the x
+  // and y sweeps, y for the z sweep)
+  const cuuint32_t q = (cuuint32_t)(8 / parts);
   const cuuint32_t box_in[3][3] = {{8, 8, q}, {8, 8, q}, {8, q, 8}};
   const cuuint32_t box_slab[3][3] = {{4, 8, q}, {8, 4, q}, {8, q, 4}};
   for (int par = 0; par < 2; ++par)
@@ -586,6 +586,7 @@ extern "C" int flash_hy_create(const flash_hy_params *params, const flash_hy_gri
   if (!amr) ALLOC(c->d_blk_nbr, (size_t)g->nblocks * 6 * sizeof(int));
   ALLOC(c->d_blk_coord, coords.size() * sizeof(int));
   ALLOC(c->d_part, g->nblocks * sizeof(CflPart));
+  if (g->ndim == 3) ALLOC(c->d_cflq, (size_t)g->nblocks * fhy::kCflParts * sizeof(fhy::CflCand));
   ALLOC(c->d_dt, sizeof(DtInfo));
   ALLOC(c->d_status, sizeof(unsigned));
   ALLOC(c->d_stepdt, sizeof(double));
@@ -647,8 +648,7 @@ extern "C" int flash_hy_create(const flash_hy_params *params, const flash_hy_gri
         }
       }
       if (ok) {
-        ALLOC(c->d_cflq, (size_t)g->nblocks * K * sizeof(fhy::CflCand));
-        c->tma_run = make_tma_maps(c, K);
+        c->tma_run = make_tma_maps(c, params->precision == FLASH_HY_PREC_MIXED ? K : fhy::kRunParts);
         if (c->tma_run)
           for (int t = 0; t < 6; ++t) {
             c->tma_run[t].runs = c->d_runs[t % 3];
@@ -1156,6 +1156,7 @@ static int enqueue_step(flash_hy_ctx *c, double dt, const int *d_list, int nlaun
   a.aux = c->aux;
   a.ncells = c->ncells;
   a.part = c->d_part;
+  a.cflq = c->d_cflq;
   a.nlaunch = nlaunch;
   a.threads = c->threads;
   a.dir_threads = c->dir_threads;
@@ -1163,7 +1164,9 @@ static int enqueue_step(flash_hy_ctx *c, double dt, const int *d_list, int nlaun
   a.sweep = c->p.precision == FLASH_HY_PREC_MIXED && c->mx_sweep == FLASH_HY_SWEEP_ZYX ? 1 : 0;
   a.stream = c->stream;
   a.tma = c->tma_maps ? c->tma_maps + 3 * c->cur : nullptr;
-  a.tma_run = c->tma_run && c->mx_runs > 1 ? c->tma_run + 3 * c->cur : nullptr;
+  // the FP64 kernels give the same bits on runs, so they always take them
+  const bool runs = c->tma_run && (c->mx_runs > 1 || c->p.precision != FLASH_HY_PREC_MIXED);
+  a.tma_run = runs ? c->tma_run + 3 * c->cur : nullptr;
   a.nblocks = c->nblocks;
   a.nlev = 0;
   int pre = 0;

@@ -124,6 +124,58 @@ __device__ __forceinline__ double div_rn(double x, double b, double rb) {
   if (a > 0x1p-960 && a < 0x1p1000 && ax > 0x1p-960 && ax < 0x1p1000) return fma(fma(-q0, b, x), rb, q0);
   return x / b;
 }
+
+// ---------------------------------------------------------------------------
+// Branch-free correctly rounded FP64 division for the direction kernels: the
+// compiler's division ends its basic block (a call for operands outside the
+// fast path), which keeps the scheduler from overlapping the forty divisions
+// of a cell.  From the mathematics of Newton's iteration and Markstein's
+// theorems (IBM J. Res. Dev. 34 (1990)):
+//   y1 = y0 (1 + e + e^2), e = 1 - b y0, from the 20-bit seed of
+//        rcp.approx.ftz.f64: within an ulp of 1 / b;
+//   y  = y1 + y1 (1 - b y1) with exact residual: RN(1 / b) unless the
+//        significand of b is all ones;
+//   q0 = RN(x y); q = q0 - y (q0 b - x) with exact residual: RN(x / b), and
+//        for b > 0 the sign of a zero x (the residual's sign is chosen so).
+// They hold where nothing leaves the normal numbers: `bad` is raised unless
+// b and x (or x = 0) lie in [2^-500, 2^500) in magnitude, and for a divisor
+// of all ones; the caller then evaluates the cell again with plain
+// divisions.  tests/test_div_rn.py checks the method against IEEE division.
+// ---------------------------------------------------------------------------
+struct Rcp { double b, r; };               // divisor (> 0) and RN(1 / b)
+// plain (Fast = false): the compiler's divisions
+template <bool Fast> struct Arith;
+template <> struct Arith<true> {
+  bool bad = false;
+  __device__ __forceinline__ void check(double x, bool when = true) {            // x = 0 or in range
+    const unsigned u = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    bad |= u - 0x20B00000u >= 0x3E800000u && u != 0u && when;
+  }
+  __device__ __forceinline__ Rcp rcp(double b, bool when = true) {
+    const unsigned hi = (unsigned)__double2hiint(b), u = hi & 0x7fffffffu;
+    bad |= (u - 0x20B00000u >= 0x3E800000u || (((hi | 0xfff00000u) & (unsigned)__double2loint(b)) == 0xffffffffu)) && when;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(b));
+    const double e = fma(-b, y, 1.0);
+    y = fma(y, fma(e, e, e), y);
+    return Rcp{b, fma(y, fma(-b, y, 1.0), y)};
+  }
+  __device__ __forceinline__ double by(double x, const Rcp &d, bool when = true) {
+    check(x, when);
+    const double q0 = x * d.r;
+    return fma(-fma(q0, d.b, -x), d.r, q0);
+  }
+  __device__ __forceinline__ double div(double x, double b, bool when = true) { return by(x, rcp(b, when), when); }
+  // x / B for a small integer constant
+  template <int B> __device__ __forceinline__ double byc(double x) { return by(x, Rcp{(double)B, 1.0 / B}); }
+};
+template <> struct Arith<false> {
+  static constexpr bool bad = false;
+  __device__ __forceinline__ Rcp rcp(double b, bool = true) { return Rcp{b, 1.0 / b}; }
+  __device__ __forceinline__ double by(double x, const Rcp &d, bool = true) { return x / d.b; }
+  __device__ __forceinline__ double div(double x, double b, bool = true) { return x / b; }
+  template <int B> __device__ __forceinline__ double byc(double x) { return x / (double)B; }
+};
 __device__ __forceinline__ double rsign(double a, double b) { return copysign(fabs(a), b); }
 __device__ __forceinline__ float rsign(float a, float b) { return copysignf(fabsf(a), b); }
 __device__ __forceinline__ double rabs(double a) { return fabs(a); }
@@ -176,14 +228,20 @@ template <class R> struct Eig {
   R cf, ahinv, a2inv, lp, rho, rp;
 };
 
+// wave speeds along DIR of a cell with sound speed e.cf
+template <class R, int DIR>
+__device__ __forceinline__ void speeds(const R *V, Eig<R> &e) {
+  const R un = V[Slots<DIR>::v1];
+  e.lam[0] = un - e.cf; e.lam[1] = un; e.lam[2] = un; e.lam[3] = un; e.lam[4] = un + e.cf;
+}
+
 template <class R, int DIR>
 __device__ __forceinline__ void eigen(const R *V, Eig<R> &e, unsigned &st) {
-  constexpr int v1 = Slots<DIR>::v1;
-  R un = V[v1];
   R a2 = V[HGC] * V[HP] / V[HD];
   if (a2 <= R(0)) st |= ST_NEG_SOUND;
   R cf = rsqrt_(a2);
-  e.lam[0] = un - cf; e.lam[1] = un; e.lam[2] = un; e.lam[3] = un; e.lam[4] = un + cf;
+  e.cf = cf;
+  speeds<R, DIR>(V, e);
   R dinv = R(1) / V[HD];
   R a2e = cf * cf;
   e.a2inv = R(1) / a2e;
@@ -192,7 +250,22 @@ __device__ __forceinline__ void eigen(const R *V, Eig<R> &e, unsigned &st) {
   e.lp = dinv * Na;
   e.rho = V[HD];
   e.rp = V[HD] * a2e;
+}
+// the same bits: g p / rho and 1 / rho share their divisor, halving is exact
+template <int DIR, class A>
+__device__ __forceinline__ void eigen64(const double *V, Eig<double> &e, A &ar, unsigned &st) {
+  const Rcp d = ar.rcp(V[HD]);
+  const double a2 = ar.by(V[HGC] * V[HP], d);
+  if (a2 <= 0.) st |= ST_NEG_SOUND;
+  const double cf = sqrt(a2);
   e.cf = cf;
+  speeds<double, DIR>(V, e);
+  const double a2e = cf * cf;
+  e.a2inv = ar.rcp(a2e).r;
+  e.ahinv = 0.5 * ar.rcp(cf).r;
+  e.lp = d.r * (0.5 * e.a2inv);
+  e.rho = V[HD];
+  e.rp = V[HD] * a2e;
 }
 
 // left eigenvector k (column k of LeftEigvec) dotted with d[0..4]
@@ -251,13 +324,33 @@ __device__ __forceinline__ void tvd_slope_d(const DevParams &P, const R *dL, con
   db[HGC] = R(0); db[HGE] = R(0);
 }
 
-template <class R, int DIR>
-__device__ __forceinline__ void tvd_slope(const DevParams &P, const R *VL, const R *V0, const R *VR,
-                                          const Eig<R> &e, R db[8]) {
-  R dL[5], dR[5];
+// FP64 with the division of the van Leer limiter through ar; the other
+// limiters have none
+template <int DIR, class A>
+__device__ __forceinline__ void tvd_slope64(const DevParams &P, const double *VL, const double *V0, const double *VR,
+                                            const Eig<double> &e, A &ar, double db[8]) {
+  double dL[5], dR[5];
 #pragma unroll
   for (int n = 0; n < 5; ++n) { dL[n] = V0[n] - VL[n]; dR[n] = VR[n] - V0[n]; }
-  tvd_slope_d<R, DIR>(P, dL, dR, V0[HEI] - VL[HEI], VR[HEI] - V0[HEI], e, db);
+  const double dLe = V0[HEI] - VL[HEI], dRe = VR[HEI] - V0[HEI];
+  if (P.limiter == 4 && P.char_limiting) {
+    auto vanleer = [&](double a, double b) {
+      const bool on = !(a * b <= 0.);
+      // a and b have one sign: take the quotient with a positive divisor
+      const double num = 2. * a * b, s = a + b;
+      const double q = ar.div(num, fabs(s), on);
+      return on ? (s < 0. ? -q : q) : 0.;
+    };
+    double d[5], t[5];
+#pragma unroll
+    for (int k = 0; k < 5; ++k) d[k] = vanleer(ldot<double, DIR>(e, k, dL), ldot<double, DIR>(e, k, dR));
+    db[HEI] = vanleer(dLe, dRe);
+    rproject<double, DIR>(e, d, t);
+#pragma unroll
+    for (int n = 0; n < 5; ++n) db[n] = t[n];
+  } else {
+    tvd_slope_d<double, DIR>(P, dL, dR, dLe, dRe, e, db);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -294,226 +387,16 @@ __device__ __forceinline__ void upwind_tflux(const DevParams &P, const R *vm1, c
 // flattening of hy_getRiemannState.F90:356-454 for the cell at stencil
 // position 3 of p[0..6] (pressures at c-3..c+3) and u[0..6] (normal vel.)
 // ---------------------------------------------------------------------------
-template <class R>
-__device__ __forceinline__ R flat_tilde(R pm2, R pm1, R pp1, R pp2, R um1, R up1) {
-  R dp1 = (pp1 - pm1);
-  R dp2 = (pp2 - pm2);
-  R dv1 = up1 - um1;
-  R Sp = rabs(dp2) > R(1.e-15) ? dp1 / dp2 - R(0.75) : R(0);
-  R ft = rmax(R(0.0), rmin(R(1.0), R(10.0) * Sp));
-  if ((rabs(dp1) / rmin(pm1, pp1) < R(1.) / R(3.)) || dv1 > R(0)) ft = R(0);
+template <class A>
+__device__ __forceinline__ double flat_tilde(A &ar, double pm2, double pm1, double pp1, double pp2, double um1,
+                                             double up1) {
+  const double dp1 = pp1 - pm1, dp2 = pp2 - pm2, dv1 = up1 - um1;
+  const bool on = fabs(dp2) > 1.e-15;
+  const double q = ar.div(dp1, fabs(dp2), on);
+  const double Sp = on ? (dp2 < 0. ? -q : q) - 0.75 : 0.;
+  double ft = rmax(0.0, rmin(1.0, 10.0 * Sp));
+  if ((ar.div(fabs(dp1), rmin(pm1, pp1)) < 1. / 3.) || dv1 > 0.) ft = 0.;
   return ft;
-}
-template <class R>
-__device__ __forceinline__ R flat_coeff(const R *p, const R *u) {
-  R t0 = flat_tilde(p[1], p[2], p[4], p[5], u[2], u[4]);
-  R dp1 = (p[4] - p[2]);
-  if (dp1 < R(0.0)) return rmax(t0, flat_tilde(p[2], p[3], p[5], p[6], u[3], u[5]));
-  if (dp1 == R(0)) return t0;
-  return rmax(t0, flat_tilde(p[0], p[1], p[3], p[4], u[1], u[3]));
-}
-
-// ---------------------------------------------------------------------------
-// hy_DataReconstructNormalDir_PPM.F90:181-842 for one cell (HLL-type
-// characteristic tracing).  V5: slots of c-2..c+2.  Outputs Wp (right face
-// state) and Wm (left face state) for slots 0..7.
-// ---------------------------------------------------------------------------
-template <class R, int DIR>
-__device__ __forceinline__ void ppm_cell(const DevParams &P, const R (*V5)[8], R flat, R dtn,
-                                         R delta, R Wp[8], R Wm[8], unsigned &st) {
-  constexpr int v1 = Slots<DIR>::v1, v2 = Slots<DIR>::v2, v3 = Slots<DIR>::v3;
-  const R *Vmm = V5[0], *Vm = V5[1], *Vc = V5[2], *Vp = V5[3], *Vpp = V5[4];
-  const R hdtn = R(0.5) * dtn;
-  Eig<R> eN, e0, eP;
-  eigen<R, DIR>(Vc, e0, st);
-  eigen<R, DIR>(Vp, eP, st);
-  eigen<R, DIR>(Vm, eN, st);
-  R dbN[8], db0[8], dbP[8];
-  tvd_slope<R, DIR>(P, Vmm, Vm, Vc, eN, dbN);
-  tvd_slope<R, DIR>(P, Vm, Vc, Vp, e0, db0);
-  tvd_slope<R, DIR>(P, Vc, Vp, Vpp, eP, dbP);
-  const R Flattening = P.use_flattening ? flat : R(0);
-
-  // slots reconstructed: 0..4 and EINT (7)
-  constexpr int NS = 6;
-  const int sl[NS] = {0, 1, 2, 3, 4, 7};
-  R vecL[8], vecR[8];
-#pragma unroll
-  for (int q = 0; q < NS; ++q) {
-    int n = sl[q];
-    vecL[n] = R(0.5) * (Vc[n] + Vm[n]) - (db0[n] - dbN[n]) / R(6.);
-    vecR[n] = R(0.5) * (Vc[n] + Vp[n]) - (dbP[n] - db0[n]) / R(6.);
-  }
-  if (P.use_steepening) {                                     // PPM.F90:639-670
-    const R eta1 = R(20.E0), eta2 = R(0.05E0), epsln = R(0.01E0), K0 = R(0.1E0);
-    R temp1 = Vp[HD] - Vm[HD];
-    if (rabs(temp1) > R(P.tiny)) {
-      R del2rhoR = (Vpp[HD] - R(2.) * Vp[HD] + Vc[HD]) / (R(6.) * delta * delta);
-      R del2rhoL = (Vc[HD] - R(2.) * Vm[HD] + Vmm[HD]) / (R(6.) * delta * delta);
-      R eta_steep = (del2rhoL - del2rhoR) * (delta * delta) / temp1;
-      if (del2rhoR * del2rhoL >= R(0)) eta_steep = R(0);
-      if (epsln * rmin(Vp[HD], Vm[HD]) - rabs(Vp[HD] - Vm[HD]) >= R(0)) eta_steep = R(0);
-      eta_steep = rmax(R(0), rmin(R(1), eta1 * (eta_steep - eta2)));
-      R temp2 = rabs(Vp[HP] - Vm[HP]) / rmin(Vp[HP], Vm[HP]);
-      R temp3 = rabs(Vp[HD] - Vm[HD]) / rmin(Vp[HD], Vm[HD]);
-      if (Vc[HGE] * K0 * temp3 - temp2 < R(0.0)) eta_steep = R(0);
-      vecL[HD] = vecL[HD] * (R(1) - eta_steep) + (Vm[HD] + R(0.5) * dbN[HD]) * eta_steep;
-      vecR[HD] = vecR[HD] * (R(1) - eta_steep) + (Vp[HD] - R(0.5) * dbP[HD]) * eta_steep;
-    }
-  }
-  if (P.use_flattening) {                                     // PPM.F90:676-679
-#pragma unroll
-    for (int q = 0; q < NS; ++q) {
-      int n = sl[q];
-      vecL[n] = Flattening * Vc[n] + (R(1.0) - Flattening) * vecL[n];
-      vecR[n] = Flattening * Vc[n] + (R(1.0) - Flattening) * vecR[n];
-    }
-  }
-  R delW[8], W6[8];
-#pragma unroll
-  for (int q = 0; q < NS; ++q) {                               // PPM.F90:686-706
-    int n = sl[q];
-    if ((vecR[n] - Vc[n]) * (Vc[n] - vecL[n]) <= R(0)) { vecL[n] = Vc[n]; vecR[n] = Vc[n]; }
-    if (R(6.) * (vecR[n] - vecL[n]) * (Vc[n] - R(0.5) * (vecL[n] + vecR[n])) > (vecR[n] - vecL[n]) * (vecR[n] - vecL[n]))
-      vecL[n] = R(3.) * Vc[n] - R(2.) * vecR[n];
-    if (R(6.) * (vecR[n] - vecL[n]) * (Vc[n] - R(0.5) * (vecL[n] + vecR[n])) < -((vecR[n] - vecL[n]) * (vecR[n] - vecL[n])))
-      vecR[n] = R(3.) * Vc[n] - R(2.) * vecL[n];
-    delW[n] = vecR[n] - vecL[n];
-    W6[n] = R(6.) * (Vc[n] - R(0.5) * (vecR[n] + vecL[n]));
-  }
-  // EINT: entropy-wave traced initial guess (PPM.F90:715-727)
-  {
-    R lmax = rmax(e0.lam[2], R(0));
-    Wp[HEI] = vecR[HEI] - lmax * hdtn * (delW[HEI] - (R(1.0) - lmax * hdtn * R(4.) / R(3.)) * W6[HEI]);
-    R lmin = -rmin(e0.lam[2], R(0));
-    Wm[HEI] = vecL[HEI] + lmin * hdtn * (delW[HEI] + (R(1.0) - lmin * hdtn * R(4.) / R(3.)) * W6[HEI]);
-  }
-  // characteristic tracing, all waves into both sides (PPM.F90:753-800)
-  R mW6[5];
-#pragma unroll
-  for (int n = 0; n < 5; ++n) mW6[n] = -W6[n];
-  R sigL[5], sigR[5];
-  const R f43 = R(4.) / R(3.);
-#pragma unroll
-  for (int n = 0; n < 5; ++n) {
-    R cA = ldot<R, DIR>(e0, n, delW);
-    R cB = ldot<R, DIR>(e0, n, mW6);
-    R lam = e0.lam[n];
-    R x = dtn * lam;
-    R AL = R(.5) * (R(-1.) - dtn * lam);
-    R BL = R(.25) * (R(1.) + R(2.) * dtn * lam + f43 * (x * x));
-    R AR = R(.5) * (R(1.) - dtn * lam);
-    R BR = R(.25) * (R(1.) - R(2.) * dtn * lam + f43 * (x * x));
-    // non-zero entries of column n of RightEigvec
-    if (n == 0 || n == 4) {
-      R rv = n == 0 ? -e0.cf : e0.cf;
-      R tL_d = AL * e0.rho * cA + BL * e0.rho * cB, tR_d = AR * e0.rho * cA + BR * e0.rho * cB;
-      R tL_v = AL * rv * cA + BL * rv * cB, tR_v = AR * rv * cA + BR * rv * cB;
-      R tL_p = AL * e0.rp * cA + BL * e0.rp * cB, tR_p = AR * e0.rp * cA + BR * e0.rp * cB;
-      if (n == 0) {
-        sigL[HD] = tL_d; sigR[HD] = tR_d; sigL[v1] = tL_v; sigR[v1] = tR_v; sigL[HP] = tL_p; sigR[HP] = tR_p;
-      } else {
-        sigL[HD] = sigL[HD] + tL_d; sigR[HD] = sigR[HD] + tR_d;
-        sigL[v1] = sigL[v1] + tL_v; sigR[v1] = sigR[v1] + tR_v;
-        sigL[HP] = sigL[HP] + tL_p; sigR[HP] = sigR[HP] + tR_p;
-      }
-    } else {
-      R tL = AL * cA + BL * cB, tR = AR * cA + BR * cB;       // reig entry 1
-      if (n == 1) { sigL[v2] = tL; sigR[v2] = tR; }
-      else if (n == 2) { sigL[HD] = sigL[HD] + tL; sigR[HD] = sigR[HD] + tR; }
-      else { sigL[v3] = tL; sigR[v3] = tR; }
-    }
-  }
-#pragma unroll
-  for (int n = 0; n < 5; ++n) {                               // PPM.F90:841-842
-    Wm[n] = Vc[n] + W6[n] / R(12.) + sigL[n];
-    Wp[n] = Vc[n] + W6[n] / R(12.) + sigR[n];
-  }
-  Wp[HGC] = Vc[HGC]; Wp[HGE] = Vc[HGE];
-  Wm[HGC] = Vc[HGC]; Wm[HGE] = Vc[HGE];
-}
-
-// ---------------------------------------------------------------------------
-// hy_prim2con.F90:37-54, hy_prim2flx.F90:49-123, hy_HLLC.F90:94-311
-// ---------------------------------------------------------------------------
-template <class R>
-__device__ __forceinline__ void prim2con(const R *V, R CU[5]) {
-  R u2 = V[HVX] * V[HVX] + V[HVY] * V[HVY] + V[HVZ] * V[HVZ];
-  CU[0] = V[HD];
-  CU[1] = V[HD] * V[HVX]; CU[2] = V[HD] * V[HVY]; CU[3] = V[HD] * V[HVZ];
-  CU[4] = R(0.5) * V[HD] * u2 + V[HP] / (V[HGE] - R(1.)) + R(0.5) * R(0.);
-}
-template <class R, int DIR>
-__device__ __forceinline__ void prim2flx(const R *V, R F[6]) {
-  constexpr int v1 = Slots<DIR>::v1;
-  R u2 = V[HVX] * V[HVX] + V[HVY] * V[HVY] + V[HVZ] * V[HVZ];
-  R E = R(0.5) * V[HD] * u2 + V[HP] / (V[HGE] - R(1.));
-  F[5] = V[HP];
-  F[0] = V[HD] * V[v1];
-  F[1] = F[0] * V[HVX];
-  F[2] = F[0] * V[HVY];
-  F[3] = F[0] * V[HVZ];
-  F[DIR] = F[DIR] + R(1.0) * V[HP];            // hy_fPresInMomFlux = 1
-  F[4] = (E + V[HP]) * V[v1];
-}
-template <class R, int DIR>
-__device__ __forceinline__ void hllc(const DevParams &P, const R *Vm, const R *Vp, R Fs[6], unsigned &st) {
-  constexpr int v1 = Slots<DIR>::v1;
-  const R tiny = R(P.tiny);
-  R velNL = Vm[v1], velNR = Vp[v1];
-  R aL2 = Vm[HGC] * Vm[HP] / Vm[HD];
-  R aR2 = Vp[HGC] * Vp[HP] / Vp[HD];
-  if ((Vm[HD] < tiny && Vm[HD] > R(0)) || (Vp[HD] < tiny && Vp[HD] > R(0)) ||
-      (Vm[HP] < tiny && Vm[HP] > R(0)) || (Vp[HP] < tiny && Vp[HP] > R(0))) {
-#pragma unroll
-    for (int n = 0; n < 6; ++n) Fs[n] = R(0);
-    return;
-  }
-  if (aL2 < R(0) || aR2 < R(0)) {
-    st |= ST_NEG_SOUND;
-#pragma unroll
-    for (int n = 0; n < 6; ++n) Fs[n] = R(0);
-    return;
-  }
-  R cfL = rsqrt_(aL2), cfR = rsqrt_(aR2);
-  R SL = rmin(velNL - cfL, velNR - cfR);
-  R SR = rmax(velNL + cfL, velNR + cfR);
-  R pL = Vm[HP], pR = Vp[HP];
-  R UL[5], UR[5], FL[6], FR[6];
-  prim2con(Vm, UL); prim2con(Vp, UR);
-  prim2flx<R, DIR>(Vm, FL); prim2flx<R, DIR>(Vp, FR);
-  R qStar = (Vp[HD] * velNR * (SR - velNR) - Vm[HD] * velNL * (SL - velNL) + pL - pR - R(0.) * R(0.) + R(0.) * R(0.));
-  qStar = qStar / (Vp[HD] * (SR - velNR) - Vm[HD] * (SL - velNL));
-  R numerL = SL - velNL, denomL = SL - qStar;
-  R numerR = SR - velNR, denomR = SR - qStar;
-  R pStar = Vm[HD] * numerL * (qStar - velNL) + pL;
-  if (SL >= R(0)) {
-#pragma unroll
-    for (int n = 0; n < 6; ++n) Fs[n] = FL[n];
-  } else if ((SL < R(0)) && (qStar >= R(0))) {
-    R dStarL = UL[0] * numerL / denomL;
-    R UC[5];
-    UC[0] = dStarL;
-    UC[4] = UL[4] * numerL / denomL + ((pStar * qStar - pL * velNL)) / denomL;
-#pragma unroll
-    for (int m = 1; m <= 3; ++m) UC[m] = (m == DIR) ? dStarL * qStar : UL[m] * numerL / denomL;
-#pragma unroll
-    for (int n = 0; n < 5; ++n) Fs[n] = FL[n] + SL * (UC[n] - UL[n]);
-    Fs[5] = FL[5];
-  } else if ((qStar < R(0)) && (SR >= R(0))) {
-    R dStarR = UR[0] * numerR / denomR;
-    R UC[5];
-    UC[0] = dStarR;
-    UC[4] = UR[4] * numerR / denomR + ((pStar * qStar - pR * velNR)) / denomR;
-#pragma unroll
-    for (int m = 1; m <= 3; ++m) UC[m] = (m == DIR) ? dStarR * qStar : UR[m] * numerR / denomR;
-#pragma unroll
-    for (int n = 0; n < 5; ++n) Fs[n] = FR[n] + SR * (UC[n] - UR[n]);
-    Fs[5] = FR[5];
-  } else {
-#pragma unroll
-    for (int n = 0; n < 6; ++n) Fs[n] = FR[n];
-  }
 }
 
 }  // namespace fhy

@@ -101,6 +101,12 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
+// L2 prefetch of [p, p + bytes) as one bulk request (16-byte aligned,
+// bytes a multiple of 16)
+__device__ __forceinline__ void bulk_prefetch_l2(const void *p, unsigned bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // The source blocks of a block's guard cells on a uniform grid: entry
 // (cz * 3 + cy) * 3 + cx for the side (0 below, 1 inside, 2 above) of each
 // coordinate; threads 0..3^NDIM-1 write one entry each.
@@ -185,14 +191,13 @@ __device__ __forceinline__ int3 blk_coords(const DevParams &P, int b) {
 // path carries the relative precision of the differences, not of the values.
 template <class R, int DIR>
 __device__ __forceinline__ void sig_dir(const DevParams &P, const double *Vm, const double *Vc, const double *Vp,
-                                        R sig[8], unsigned &st) {
+                                        Eig<R> e, R sig[8]) {
   R c[8], dl[5], dr[5];
 #pragma unroll
   for (int n = 0; n < 8; ++n) c[n] = R(Vc[n]);
 #pragma unroll
   for (int n = 0; n < 5; ++n) { dl[n] = R(Vc[n] - Vm[n]); dr[n] = R(Vp[n] - Vc[n]); }
-  Eig<R> e;
-  eigen<R, DIR>(c, e, st);
+  speeds<R, DIR>(c, e);
   upwind_tflux_d<R, DIR>(P, dl, dr, R(Vc[HEI] - Vm[HEI]), R(Vp[HEI] - Vc[HEI]), e, sig);
 }
 
@@ -265,26 +270,6 @@ __device__ __forceinline__ void staged_prim(const DevParams &P, const double *sQ
   V[HGC] = P.gamma; V[HGE] = GAME ? p / (eg * rho) + 1 : 0.0; V[HEI] = eg;
 }
 
-// The lines of interior cells along DIR with four cells beyond the block on
-// either side (the stencil of the FP64 direction kernel: PPM +-2, the
-// flattening's pressures +-3 around line cells [-1, N]), in the thread
-// order of the line cells.
-template <int NDIM, int NX, int NY, int NZ, int DIR>
-struct LineStage {
-  static constexpr int sx = DIR == 1 ? NX + 8 : NX, sy = NDIM > 1 ? (DIR == 2 ? NY + 8 : NY) : 1,
-                       sz = NDIM > 2 ? (DIR == 3 ? NZ + 8 : NZ) : 1;
-  static constexpr int n = sx * sy * sz;
-  static constexpr int step = DIR == 1 ? 1 : (DIR == 2 ? sx : sx * sy);
-  __device__ static __forceinline__ int idx(int i, int j, int k) {
-    return ((k + 4 * (DIR == 3)) * sy + (j + 4 * (DIR == 2))) * sx + (i + 4 * (DIR == 1));
-  }
-  __device__ static __forceinline__ void decode(int c, int &i, int &j, int &k) {
-    i = c % sx - 4 * (DIR == 1);
-    j = NDIM > 1 ? (c / sx) % sy - 4 * (DIR == 2) : 0;
-    k = NDIM > 2 ? c / (sx * sy) - 4 * (DIR == 3) : 0;
-  }
-};
-
 template <int NDIM, int NX, int NY, int NZ>
 struct SigStage {
   using E = Ext<NDIM, NX, NY, NZ, 2>;
@@ -329,15 +314,26 @@ __global__ void __launch_bounds__(320, NDIM > 2 ? (sizeof(R) == 4 ? 3 : 2) : 1) 
     const int e = E::idx(i, j, k);
     double Vc[8], Vm[8], Vp[8];
     staged_prim(P, sQ, E::n, e, Vc);
+    Eig<R> eg;                               // one for the directions, which differ in the wave speeds only
+    if constexpr (sizeof(R) == 8) {
+      Arith<true> ar;
+      eigen64<1>(Vc, eg, ar, st);
+      if (ar.bad) { Arith<false> plain; eigen64<1>(Vc, eg, plain, st); }
+    } else {
+      R c[8];
+#pragma unroll
+      for (int n = 0; n < 8; ++n) c[n] = R(Vc[n]);
+      eigen<R, 1>(c, eg, st);
+    }
 #pragma unroll
     for (int d = 1; d <= NDIM; ++d) {
       const int es = d == 1 ? 1 : (d == 2 ? E::ex : E::ex * E::ey);
       staged_prim(P, sQ, E::n, e - es, Vm);
       staged_prim(P, sQ, E::n, e + es, Vp);
       R s[8];
-      if (d == 1) sig_dir<R, 1>(P, Vm, Vc, Vp, s, st);
-      else if (d == 2) sig_dir<R, 2>(P, Vm, Vc, Vp, s, st);
-      else sig_dir<R, 3>(P, Vm, Vc, Vp, s, st);
+      if (d == 1) sig_dir<R, 1>(P, Vm, Vc, Vp, eg, s);
+      else if (d == 2) sig_dir<R, 2>(P, Vm, Vc, Vp, eg, s);
+      else sig_dir<R, 3>(P, Vm, Vc, Vp, eg, s);
       R *dst = SIG + ((size_t)(P.slot ? P.slot[b] : (int)blockIdx.x) * NDIM + (d - 1)) * 6 * B::n + t;
 #pragma unroll
       for (int q = 0; q < 6; ++q) dst[(size_t)q * B::n] = s[sig_slot(q)];
@@ -394,6 +390,57 @@ __device__ void cfl_block_reduce(CflCand c, int blk, double cfl, CflPart *part) 
   }
 }
 
+// the CTA's candidates of the K blocks it holds part of, one to at(m) for
+// block m; merged per block by k_cfl_merge (one barrier: every warp reduces
+// its K candidates, then thread m merges the warps' candidates of block m)
+template <int K, class At>
+__device__ __forceinline__ void cfl_parts_reduce(const CflCand (&cand)[K], At at) {
+  __shared__ CflCand red[32][K];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int m = 0; m < K; ++m) {
+    CflCand c = cand[m];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      CflCand b;
+      b.key = __shfl_down_sync(0xffffffffu, c.key, o);
+      b.val = __shfl_down_sync(0xffffffffu, c.val, o);
+      b.idx = __shfl_down_sync(0xffffffffu, c.idx, o);
+      if (lane + o < 32) cfl_merge(c, b);
+    }
+    if (lane == 0) red[w][m] = c;
+  }
+  __syncthreads();
+  if (threadIdx.x < K) {
+    const int m = threadIdx.x;
+    CflCand a = red[0][m];
+    for (int q = 1; q < (int)(blockDim.x + 31) / 32; ++q) cfl_merge(a, red[q][m]);
+    *at(m) = a;
+  }
+}
+
+// Per block (of the list, or all), the K candidates of the CTAs that share
+// it merged into the block's CFL result, as cfl_block_reduce writes it for a
+// block handled whole (Hydro_computeDt.F90:265-284).
+template <int NX, int NY, int K>
+__global__ void k_cfl_merge(const CflCand *cq, const int *list, int n, double cfl, CflPart *part) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const int b = list ? list[t] : t;
+  CflCand a = cq[(size_t)b * K];
+#pragma unroll
+  for (int q = 1; q < K; ++q) cfl_merge(a, cq[(size_t)b * K + q]);
+  CflPart r;
+  if (a.key > 0.0) {
+    r.dt = cfl / a.val;
+    r.i = a.idx % NX; r.j = (a.idx / NX) % NY; r.k = a.idx / (NX * NY);
+  } else {
+    r.dt = DBL_MAX; r.i = r.j = r.k = -1;
+  }
+  r.blk = b;
+  part[b] = r;
+}
+
 // ---------------------------------------------------------------------------
 // exact Riemann face flux (no FLASH5 counterpart; Toro ch. 4, exact_rs.cuh)
 // ---------------------------------------------------------------------------
@@ -444,15 +491,18 @@ __device__ __forceinline__ void exact_face(const DevParams &P, const xrs::Gas &G
 // The register of nv flux components per face: reg[(slot * 2 NDIM + face
 // side) * NF * nv + face * nv + v]; the hydro's is P.freg with the NFLX
 // fluxes, the species pass keeps one register per species.
-template <int NDIM, int NX, int NY, int NZ, int DIR, class FaceIdx>
-__device__ void flux_register_v(const DevParams &P, int b, int3 bc, double *sF, int fstride, FaceIdx fidx,
+// With Q > 1 the CTA holds part `part` of the block's faces: their slower
+// tangential coordinate split into Q ranges (fidx takes it relative to its
+// range).
+template <int NDIM, int NX, int NY, int NZ, int DIR, int Q = 1, class FaceIdx>
+__device__ void flux_register_v(const DevParams &P, int b, int3 bc, int part, double *sF, int fstride, FaceIdx fidx,
                                 double *reg, int nv) {
   constexpr int N = DIR == 1 ? NX : (DIR == 2 ? NY : NZ);
   constexpr int n1 = DIR == 1 ? NY : NX;
   constexpr int n2 = NDIM > 2 ? (DIR == 3 ? NY : NZ) : 1;
-  constexpr int NF = n1 * n2;
+  constexpr int NF = n1 * n2, NFQ = NF / Q, n2q = n2 / Q;
   constexpr int T1 = DIR == 1 ? 1 : 0, T2 = DIR == 3 ? 1 : 2;
-  const int l = P.blk_level[b];
+  const int l = P.blk_level[b], t20 = part * n2q;
   for (int s = 0; s < 2; ++s) {
     int pos[3] = {bc.x, bc.y, NDIM > 2 ? bc.z : 0};
     pos[DIR - 1] += s ? 1 : -1;
@@ -465,14 +515,14 @@ __device__ void flux_register_v(const DevParams &P, int b, int3 bc, double *sF, 
     const int along = s ? N : 0;
     if (m < 0) {
       double *dst = reg + ((size_t)P.slot[b] * 2 * NDIM + 2 * (DIR - 1) + s) * NF * nv;
-      for (int q = threadIdx.x; q < NF * nv; q += blockDim.x) {
+      for (int q = threadIdx.x; q < NFQ * nv; q += blockDim.x) {
         const int face = q / nv, v = q % nv;
-        dst[q] = sF[v * fstride + fidx(along, face % n1, face / n1)];
+        dst[q + t20 * n1 * nv] = sF[v * fstride + fidx(along, face % n1, face / n1)];
       }
     } else if (!P.leaf[m]) {
       const double w = NDIM > 2 ? 0.25 : 0.5;
-      for (int q = threadIdx.x; q < NF * nv; q += blockDim.x) {
-        const int face = q / nv, v = q % nv, q1 = face % n1, q2 = face / n1;
+      for (int q = threadIdx.x; q < NFQ * nv; q += blockDim.x) {
+        const int face = q / nv, v = q % nv, q1 = face % n1, q2 = face / n1 + t20;
         int o[3] = {0, 0, 0};
         o[DIR - 1] = s ? 0 : 1;
         o[T1] = q1 >= n1 / 2;
@@ -485,16 +535,16 @@ __device__ void flux_register_v(const DevParams &P, int b, int3 bc, double *sF, 
             const int f1 = 2 * (q1 - o[T1] * (n1 / 2)) + r1, f2 = NDIM > 2 ? 2 * (q2 - o[T2] * (n2 / 2)) + r2 : 0;
             acc = acc + w * src[(f1 + n1 * f2) * nv + v];
           }
-        sF[v * fstride + fidx(along, q1, q2)] = acc;
+        sF[v * fstride + fidx(along, q1, q2 - t20)] = acc;
       }
     }
   }
 }
 
-template <int NDIM, int NX, int NY, int NZ, int DIR, class FaceIdx>
-__device__ __forceinline__ void flux_register(const DevParams &P, int b, int3 bc, double *sF, int fstride,
+template <int NDIM, int NX, int NY, int NZ, int DIR, int Q = 1, class FaceIdx>
+__device__ __forceinline__ void flux_register(const DevParams &P, int b, int3 bc, int part, double *sF, int fstride,
                                               FaceIdx fidx) {
-  flux_register_v<NDIM, NX, NY, NZ, DIR>(P, b, bc, sF, fstride, fidx, P.freg, NFLX);
+  flux_register_v<NDIM, NX, NY, NZ, DIR, Q>(P, b, bc, part, sF, fstride, fidx, P.freg, NFLX);
 }
 
 // ---------------------------------------------------------------------------
@@ -523,41 +573,57 @@ __device__ __forceinline__ void face_coords(int f, int &along, int &t1, int &t2)
   t2 = DIR == 3 ? j : k;
 }
 
+// whether the face or cell with slower tangential coordinate t2 lies in part
+// `part` of Q; t2 becomes relative to the part
+template <int NDIM, int NY, int NZ, int DIR, int Q>
+__device__ __forceinline__ bool in_part(int part, int &t2) {
+  constexpr int n2q = (NDIM > 2 ? (DIR == 3 ? NY : NZ) : 1) / Q;
+  if (Q == 1) return true;
+  t2 -= part * n2q;
+  return t2 >= 0 && t2 < n2q;
+}
+
 // store: sF faces and the cell pressure sums (sp(t) for a cell position t)
-template <int NDIM, int NX, int NY, int NZ, int DIR, class T, class FaceIdx, class CellSp>
-__device__ void flux_store(const DevParams &P, int b, const T *sF, int fstride, FaceIdx fidx, CellSp sp) {
+template <int NDIM, int NX, int NY, int NZ, int DIR, int Q = 1, class FaceIdx, class CellSp>
+__device__ void flux_store(const DevParams &P, int b, int part, const double *sF, int fstride, FaceIdx fidx,
+                           CellSp sp) {
   using FS = FluxStore<NDIM, NX, NY, NZ>;
   double *o = FS::base(P, b, DIR);
   for (int q = threadIdx.x; q < NFLX * FS::NF; q += blockDim.x) {
     const int v = q / FS::NF, f = q % FS::NF;
     int a, t1, t2;
     face_coords<NDIM, NX, NY, NZ, DIR>(f, a, t1, t2);
-    o[q] = double(sF[v * fstride + fidx(a, t1, t2)]);
+    if (in_part<NDIM, NY, NZ, DIR, Q>(part, t2)) o[q] = sF[v * fstride + fidx(a, t1, t2)];
   }
   for (int c = threadIdx.x; c < FS::NCB; c += blockDim.x) {
     const int i = c % NX, j = (c / NX) % NY, k = c / (NX * NY);
-    const int a = DIR == 1 ? i : (DIR == 2 ? j : k), t1 = DIR == 1 ? j : i, t2 = DIR == 3 ? j : k;
-    o[NFLX * FS::NF + c] = sp(fidx(a, t1, t2));
+    const int a = DIR == 1 ? i : (DIR == 2 ? j : k), t1 = DIR == 1 ? j : i;
+    int t2 = DIR == 3 ? j : k;
+    if (in_part<NDIM, NY, NZ, DIR, Q>(part, t2)) o[NFLX * FS::NF + c] = sp(fidx(a, t1, t2));
   }
 }
 
-// ---------------------------------------------------------------------------
-// k_dir: one direction of the unsplit update for one block per CTA.
-//   phase 1: face states W-/W+ of the line cells (c_DIR in [-1, N], other
-//            coordinates interior) -- PPM (hy_dataReconstOneStep.F90:485-
-//            716), transverse corrections (:918-951), last negativity
-//            check (:1120-1154), 3D full-CTU cross terms and positivity
-//            fallback (hy_getRiemannState.F90:956-1313)
-//   phase 2: HLLC (RS = 0) or the exact solver (RS = 1) at the N+1 faces
-//            of every line plus the auxiliary
-//            internal-energy and volume fluxes (hy_getFaceFlux.F90:283-442)
-//   phase 3: accumulation of the conservative update in direction order
-//            x, y, z (updateConservedVariable, hy_unsplitUpdate.F90:1187-
-//            1242); the last direction finishes the cell: internal-energy
-//            update with the n+1/2 pressure (:657-672, hy_getFaceFlux.F90:
-//            551-557 and y/z analogues), hy_energyFix (:188-253), the EOS
-//            and the CFL reduction (Hydro_computeDt.F90:186-290).
-// ---------------------------------------------------------------------------
+// replay: the stored faces into sF, the cell pressure sums through sp(t, sum)
+template <int NDIM, int NX, int NY, int NZ, int DIR, int Q = 1, class FaceIdx, class CellSp>
+__device__ void flux_load(const DevParams &P, int b, int part, double *sF, int fstride, FaceIdx fidx, CellSp sp) {
+  using FS = FluxStore<NDIM, NX, NY, NZ>;
+  const double *src = FS::base(P, b, DIR);
+  for (int q = threadIdx.x; q < NFLX * FS::NF; q += blockDim.x) {
+    const int v = q / FS::NF, f = q % FS::NF;
+    int a, t1, t2;
+    face_coords<NDIM, NX, NY, NZ, DIR>(f, a, t1, t2);
+    if (in_part<NDIM, NY, NZ, DIR, Q>(part, t2)) sF[v * fstride + fidx(a, t1, t2)] = src[q];
+  }
+  for (int c = threadIdx.x; c < FS::NCB; c += blockDim.x) {
+    const int i = c % NX, j = (c / NX) % NY, k = c / (NX * NY);
+    const int a = DIR == 1 ? i : (DIR == 2 ? j : k), t1 = DIR == 1 ? j : i;
+    int t2 = DIR == 3 ? j : k;
+    if (in_part<NDIM, NY, NZ, DIR, Q>(part, t2)) sp(fidx(a, t1, t2), src[NFLX * FS::NF + c]);
+  }
+}
+
+// Line cells of a direction (c_DIR in [-1, N], other coordinates interior):
+// the order in which the hydro kernels leave the species' per-line data.
 template <int NDIM, int NX, int NY, int NZ, class R, int DIR>
 struct DirGeom {
   static constexpr int rx = DIR == 1 ? NX + 2 : NX;
@@ -576,325 +642,12 @@ struct DirGeom {
   __device__ static __forceinline__ int idx(int i, int j, int k) {
     return ((k + (DIR == 3)) * ry + (j + (DIR == 2))) * rx + (i + (DIR == 1));
   }
-  static constexpr size_t smem_bytes() { return (size_t)n * (14 + NFLX) * sizeof(R); }
 };
 // per-slot offset of a direction's line cells in sp_mf / sp_fb
 template <int NDIM, int NX, int NY, int NZ, int DIR>
 __device__ __forceinline__ size_t sp_line_base(int slot) {
   using L = DirGeom<NDIM, NX, NY, NZ, double, DIR>;
   return ((size_t)slot * NDIM + (DIR - 1)) * L::n;
-}
-
-// slots stored for the face states: dens, velx, vely, velz, pres, game, eint
-__device__ __forceinline__ int wslot(int q) { return q < 5 ? q : q + 1; }
-
-template <int NDIM, int NX, int NY, int NZ, class R, int DIR, bool FIRST, bool LAST, int VAR, int RS>
-__global__ void __launch_bounds__(320) k_dir(const DevParams P, const R *__restrict__ SIG, double *__restrict__ ACC,
-                                             double *__restrict__ AUX, size_t ncells, CflPart *part) {
-  using G = DirGeom<NDIM, NX, NY, NZ, R, DIR>;
-  using B = Box<NDIM, NX, NY, NZ>;
-  constexpr int NCB = NX * NY * NZ;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  R *sWp = reinterpret_cast<R *>(smem_raw);     // [7][n]
-  R *sWm = sWp + 7 * G::n;                       // [7][n]
-  R *sF = sWm + 7 * G::n;                        // [8][n]
-  const int b = P.blk_list ? P.blk_list[blockIdx.x] : blockIdx.x;
-  const int3 bc = blk_coords(P, b);
-  unsigned st = 0;
-  const double dt = P.dt_dev ? *P.dt_dev : P.dt;
-  double del[3];
-  blk_deltas(P, b, del);
-  const double delta = del[DIR - 1];
-  const R dtn = R(dt / delta);
-  const R hdtx = R(0.5 * dt / del[0]), hdty = R(0.5 * dt / del[1]), hdtz = R(0.5 * dt / del[2]);
-  const R *sigb = SIG + (size_t)(P.slot ? P.slot[b] : (int)blockIdx.x) * NDIM * 6 * B::n;
-
-  auto fidx = [](int along, int t1, int t2) {
-    const int i = DIR == 1 ? along : t1, j = DIR == 1 ? t1 : (DIR == 2 ? along : t2),
-              k = DIR == 3 ? along : (NDIM > 2 ? t2 : 0);
-    return ((k + (DIR == 3)) * G::ry + (j + (DIR == 2))) * G::rx + (i + (DIR == 1));
-  };
-  if (P.fmode != 3) {
-  // ---------------- phase 0: the stencil of every line, staged once ---------
-  // (in the flux array, unused until phase 2: 5 (N+8) <= 8 (N+2) for N >= 8)
-  using LS = LineStage<NDIM, NX, NY, NZ, DIR>;
-  static_assert(5 * LS::n <= NFLX * G::n, "line stage fits the flux array");
-  __shared__ int sNb[NDIM > 2 ? 27 : 9];
-  double *sQ = reinterpret_cast<double *>(sF);
-  if (P.lh == nullptr) {
-    neighbour_table<NDIM, NX, NY, NZ>(P, bc, sNb);
-    __syncthreads();
-  }
-  stage_prims<NDIM, NX, NY, NZ>(P, b, bc, P.slot ? P.slot[b] : (int)blockIdx.x, sNb, sQ, LS::n,
-                                [](int c, int &i, int &j, int &k) {
-                                  LS::decode(c, i, j, k);
-                                  return true;
-                                });
-  __syncthreads();
-  // ---------------- phase 1: face states of the line cells ----------------
-  for (int t = threadIdx.x; t < G::n; t += blockDim.x) {
-    int i, j, k;
-    G::decode(t, i, j, k);
-    const int e0 = LS::idx(i, j, k);
-    R V5[5][8];
-    double Vd[8];
-#pragma unroll
-    for (int s = -2; s <= 2; ++s) {
-      if (s == 0) staged_prim<true>(P, sQ, LS::n, e0, Vd);
-      else staged_prim<false>(P, sQ, LS::n, e0 + s * LS::step, Vd);
-#pragma unroll
-      for (int n = 0; n < 8; ++n) V5[s + 2][n] = R(Vd[n]);
-    }
-    R flat = R(0);
-    if (P.use_flattening) {
-      R p7[7], u7[7];
-      const int em = e0 - 3 * LS::step, ep = e0 + 3 * LS::step;
-      p7[0] = R(sQ[em] * sQ[4 * LS::n + em] * P.gam1inv);
-      p7[6] = R(sQ[ep] * sQ[4 * LS::n + ep] * P.gam1inv);
-#pragma unroll
-      for (int s = 0; s < 5; ++s) { p7[s + 1] = V5[s][HP]; u7[s + 1] = V5[s][Slots<DIR>::v1]; }
-      u7[0] = R(0); u7[6] = R(0);
-      flat = flat_coeff(p7, u7);
-    }
-    if (P.sp_flat) P.sp_flat[sp_line_base<NDIM, NX, NY, NZ, DIR>(P.slot ? P.slot[b] : (int)blockIdx.x) + t] = double(flat);
-    R Wp[8], Wm[8];
-    ppm_cell<R, DIR>(P, V5, flat, dtn, R(delta), Wp, Wm, st);
-    const R *Vc = V5[2];
-    // transverse corrections with the sig of the other directions (same cell)
-    const int bi = B::idx(i, j, k);
-    R sx[8], sy[8], sz[8];
-    if (DIR != 1) load_sig(sigb + 0 * 6 * B::n + bi, B::n, sx);
-    if (NDIM > 1 && DIR != 2) load_sig(sigb + 1 * 6 * B::n + bi, B::n, sy);
-    if (NDIM > 2 && DIR != 3) load_sig(sigb + 2 * 6 * B::n + bi, B::n, sz);
-    const int sl[6] = {0, 1, 2, 3, 4, 7};
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-      int n = sl[q];
-      if (NDIM == 2) {
-        if (DIR == 1) { Wm[n] = Wm[n] - hdty * sy[n]; Wp[n] = Wp[n] - hdty * sy[n]; }
-        else          { Wm[n] = Wm[n] - hdtx * sx[n]; Wp[n] = Wp[n] - hdtx * sx[n]; }
-      } else {
-        if (DIR == 1)      { Wm[n] = Wm[n] - hdty * sy[n] - hdtz * sz[n]; Wp[n] = Wp[n] - hdty * sy[n] - hdtz * sz[n]; }
-        else if (DIR == 2) { Wm[n] = Wm[n] - hdtx * sx[n] - hdtz * sz[n]; Wp[n] = Wp[n] - hdtx * sx[n] - hdtz * sz[n]; }
-        else               { Wm[n] = Wm[n] - hdtx * sx[n] - hdty * sy[n]; Wp[n] = Wp[n] - hdtx * sx[n] - hdty * sy[n]; }
-      }
-    }
-    if (Wm[HD] < R(0) || Wp[HD] < R(0) || Wm[HP] < R(0) || Wp[HP] < R(0)) {
-#pragma unroll
-      for (int n = 0; n < 8; ++n) { Wm[n] = Vc[n]; Wp[n] = Vc[n]; }
-    }
-    if (NDIM == 3 && P.use_ctu) {
-      // axis / sig direction pairs of hy_getRiemannState.F90:999-1022,
-      // 1101-1124, 1204-1227
-      constexpr int A1 = DIR == 1 ? 2 : (DIR == 2 ? 3 : 1), S1 = DIR == 1 ? 3 : (DIR == 2 ? 1 : 2);
-      constexpr int A2 = DIR == 1 ? 3 : (DIR == 2 ? 1 : 2), S2 = DIR == 1 ? 2 : (DIR == 2 ? 3 : 1);
-      const double dA = del[A1 - 1], dB = del[A2 - 1];
-      const R fac = R(dt * dt / (6. * (DIR == 1 ? del[1] : (DIR == 2 ? del[2] : del[0])) *
-                                 (DIR == 1 ? del[2] : (DIR == 2 ? del[0] : del[1]))));
-      (void)dA; (void)dB;
-      R T1[8], T2[8];
-      {
-        R sm[8], s0[8], sp[8];
-        const R *base = sigb + (size_t)(S1 - 1) * 6 * B::n;
-        load_sig(base + B::idx(i - (A1 == 1), j - (A1 == 2), k - (A1 == 3)), B::n, sm);
-        load_sig(base + bi, B::n, s0);
-        load_sig(base + B::idx(i + (A1 == 1), j + (A1 == 2), k + (A1 == 3)), B::n, sp);
-        Eig<R> e;
-        eigen<R, A1>(Vc, e, st);
-        upwind_tflux<R, A1>(P, sm, s0, sp, e, T1);
-      }
-      {
-        R sm[8], s0[8], sp[8];
-        const R *base = sigb + (size_t)(S2 - 1) * 6 * B::n;
-        load_sig(base + B::idx(i - (A2 == 1), j - (A2 == 2), k - (A2 == 3)), B::n, sm);
-        load_sig(base + bi, B::n, s0);
-        load_sig(base + B::idx(i + (A2 == 1), j + (A2 == 2), k + (A2 == 3)), B::n, sp);
-        Eig<R> e;
-        eigen<R, A2>(Vc, e, st);
-        upwind_tflux<R, A2>(P, sm, s0, sp, e, T2);
-      }
-#pragma unroll
-      for (int q = 0; q < 6; ++q) {
-        int n = sl[q];
-        Wp[n] = Wp[n] + (T1[n] + T2[n]) * fac;
-        Wm[n] = Wm[n] + (T1[n] + T2[n]) * fac;
-      }
-      const bool fb = Wp[HD] <= R(0) || Wm[HD] <= R(0) || Wp[HP] <= R(0) || Wm[HP] <= R(0);
-      if (fb) {
-#pragma unroll
-        for (int n = 0; n < 8; ++n) { Wm[n] = Vc[n]; Wp[n] = Vc[n]; }
-      }
-      if (P.sp_fb) P.sp_fb[sp_line_base<NDIM, NX, NY, NZ, DIR>(P.slot ? P.slot[b] : (int)blockIdx.x) + t] = fb;
-    }
-#pragma unroll
-    for (int q = 0; q < 7; ++q) {
-      sWp[q * G::n + t] = Wp[wslot(q)];
-      sWm[q * G::n + t] = Wm[wslot(q)];
-    }
-  }
-  __syncthreads();
-
-  // ---------------- phase 2: Riemann problems at the faces ----------------
-  const R gam = R(P.gamma);
-  for (int t = threadIdx.x; t < G::n; t += blockDim.x) {
-    int i, j, k;
-    G::decode(t, i, j, k);
-    if (G::along(i, j, k) < 0) continue;
-    R VL[8], VR[8];
-#pragma unroll
-    for (int q = 0; q < 7; ++q) {
-      VL[wslot(q)] = sWp[q * G::n + t - G::stride];
-      VR[wslot(q)] = sWm[q * G::n + t];
-    }
-    VL[HGC] = gam; VR[HGC] = gam;
-    R F[6];
-    if constexpr (RS == 1) exact_face<DIR>(P, P.gas, VL, VR, F, st);
-    else hllc<R, DIR>(P, VL, VR, F, st);
-#pragma unroll
-    for (int n = 0; n < 6; ++n) sF[n * G::n + t] = F[n];
-    R fv = R(0), fe = R(0);
-    if (P.use_aux_eint) {                         // hy_getFaceFlux.F90:433-442
-      if (F[FDENS] > R(0)) { fv = F[FDENS] / VL[HD]; fe = F[FDENS] * VL[HEI]; }
-      else { fv = F[FDENS] / VR[HD]; fe = F[FDENS] * VR[HEI]; }
-    }
-    sF[FEINT * G::n + t] = fe;
-    sF[FVOLU * G::n + t] = fv;
-    if (P.sp_mf) P.sp_mf[sp_line_base<NDIM, NX, NY, NZ, DIR>(P.slot ? P.slot[b] : (int)blockIdx.x) + t] = double(F[FDENS]);
-  }
-  __syncthreads();
-  if constexpr (sizeof(R) == 8) {
-    if (P.freg) {       // AMR: fine/coarse faces
-      flux_register<NDIM, NX, NY, NZ, DIR>(P, b, bc, sF, G::n, [](int along, int t1, int t2) {
-        const int i = DIR == 1 ? along : t1, j = DIR == 1 ? t1 : (DIR == 2 ? along : t2),
-                  k = DIR == 3 ? along : (NDIM > 2 ? t2 : 0);
-        return ((k + (DIR == 3)) * G::ry + (j + (DIR == 2))) * G::rx + (i + (DIR == 1));
-      });
-      __syncthreads();
-    }
-  }
-
-  } else {
-    // replay: the stored fluxes, and the stored pressure sums in place of
-    // the face-state sum N05 + P05 of phase 3
-    using FS = FluxStore<NDIM, NX, NY, NZ>;
-    const double *src = FS::base(P, b, DIR);
-    for (int q = threadIdx.x; q < NFLX * FS::NF; q += blockDim.x) {
-      const int v = q / FS::NF, f = q % FS::NF;
-      int a, t1, t2;
-      face_coords<NDIM, NX, NY, NZ, DIR>(f, a, t1, t2);
-      sF[v * G::n + fidx(a, t1, t2)] = R(src[q]);
-    }
-    for (int c = threadIdx.x; c < FS::NCB; c += blockDim.x) {
-      const int i = c % NX, j = (c / NX) % NY, k = c / (NX * NY);
-      const int t = fidx(DIR == 1 ? i : (DIR == 2 ? j : k), DIR == 1 ? j : i, DIR == 3 ? j : k);
-      sWm[4 * G::n + t] = R(src[NFLX * FS::NF + c]);
-      sWp[4 * G::n + t] = R(0);
-    }
-    __syncthreads();
-  }
-  if (P.fmode == 1 || P.fmode == 2) {
-    flux_store<NDIM, NX, NY, NZ, DIR>(P, b, sF, G::n, fidx, [&](int t) {
-      return double(sWm[4 * G::n + t]) + double(sWp[4 * G::n + t]);
-    });
-    if (P.fmode == 2) {
-      if (st) atomicOr(P.status, st);
-      return;
-    }
-  }
-
-  // ---------------- phase 3: conservative update ----------------
-  const double dtd = dt / delta;
-  CflCand cand; cand.key = 0.0; cand.val = 0.0; cand.idx = 0x7fffffff;
-  for (int t = threadIdx.x; t < G::n; t += blockDim.x) {
-    int i, j, k;
-    G::decode(t, i, j, k);
-    int a = G::along(i, j, k);
-    if (a < 0 || a >= G::nd) continue;
-    const int loc = (k * NY + j) * NX + i;
-    const size_t off = (size_t)b * NCB + loc;
-    double FL[NFLX], FR[NFLX];
-#pragma unroll
-    for (int n = 0; n < NFLX; ++n) { FL[n] = double(sF[n * G::n + t]); FR[n] = double(sF[n * G::n + t + G::stride]); }
-    double U[5];
-    if (FIRST) {
-      double rho = P.s_in[0][off], vx = P.s_in[1][off], vy = P.s_in[2][off], vz = P.s_in[3][off], e = P.s_in[4][off];
-      double ekin = 0.5 * (vx * vx + vy * vy + vz * vz);
-      U[0] = rho; U[1] = vx * rho; U[2] = vy * rho; U[3] = vz * rho; U[4] = rho * (e + ekin);
-    } else {
-#pragma unroll
-      for (int n = 0; n < 5; ++n) U[n] = ACC[n * ncells + off];
-    }
-#pragma unroll
-    for (int n = 0; n < 5; ++n) U[n] = U[n] - dtd * (FR[n] - FL[n]);
-    const double ea = FL[FEINT] - FR[FEINT], eb = FL[FVOLU] - FR[FVOLU];
-    const double sp = double(sWm[4 * G::n + t]) + double(sWp[4 * G::n + t]);   // N05 + P05
-    if (!LAST) {
-#pragma unroll
-      for (int n = 0; n < 5; ++n) ACC[n * ncells + off] = U[n];
-      double *ax = AUX + (size_t)(DIR - 1) * 3 * ncells;
-      ax[off] = ea; ax[ncells + off] = eb; ax[2 * ncells + off] = sp;
-    } else {
-#pragma unroll
-      for (int n = 0; n < 5; ++n) U[n] = U[n] + 0.0;       // + dt*(Sgeo + Sphys), both +0 here
-      const double rho0 = P.s_in[0][off], e0 = P.s_in[4][off];
-      double IntEner = 0.0;
-      if (P.use_aux_eint) {
-        // n+1/2 pressure: scrch_Ptr(1) of hy_getFaceFlux.F90:551-557 and the
-        // y/z averages
-        double pb;
-        const double sx = AUX[2 * ncells + off];
-        if (NDIM == 2) {
-          pb = (0.5 * sx) * 0.5 + sp * 0.25;
-        } else {
-          const double sy = AUX[3 * ncells + 2 * ncells + off];
-          pb = ((0.5 * sx) * 0.5 + sy * 0.25) * 4.0;
-          pb = (pb + sp) / 6.0;
-        }
-        IntEner = rho0 * e0;
-        {
-          const double *ax = AUX;
-          IntEner = IntEner + dt / del[0] * (ax[off] + pb * ax[ncells + off]);
-        }
-        if (NDIM == 2) {
-          IntEner = IntEner + dt / del[1] * (ea + pb * eb);
-        } else {
-          const double *ay = AUX + 3 * ncells;
-          IntEner = IntEner + dt / del[1] * (ay[off] + pb * ay[ncells + off]);
-          IntEner = IntEner + dt / del[2] * (ea + pb * eb);
-        }
-        IntEner = IntEner + dt * 0.;
-      }
-      // hy_unsplitUpdate.F90:811-893
-      double dens = rmax(U[0], P.smlrho);
-      double vx = U[1] / dens, vy = U[2] / dens, vz = U[3] / dens;
-      double ener = U[4] / dens;
-      double eaux = IntEner / dens;
-      // hy_energyFix.F90:188-253
-      double ekin = 0.5 * (vx * vx + vy * vy + vz * vz);
-      double eint = ener - ekin - 0.0;
-      double newE;
-      if (!P.use_aux_eint || eint > P.eswitch * (ekin + 0.0)) newE = rmax(P.smalle, eint);
-      else newE = rmax(P.smalle, eaux);
-      ener = newE + ekin;
-      // Eos_wrapped(MODE_DENS_EI)
-      double e = newE;
-      if (ener - ekin > rmax(P.smalle, P.eswitch * ekin)) e = ener - ekin;
-      P.s_out[0][off] = dens; P.s_out[1][off] = vx; P.s_out[2][off] = vy; P.s_out[3][off] = vz;
-      P.s_out[4][off] = e;
-      if (!(isfinite(dens) && isfinite(vx) && isfinite(vy) && isfinite(vz) && isfinite(e))) st |= ST_NAN;
-      // CFL: Hydro_computeDt.F90:260-284 on the new state
-      double pres = dens * e * P.gam1inv;
-      double c2 = P.gamma * pres / dens;
-      double cs = sqrt(c2);
-      double dtl = (fabs(vx - 0.) + cs) * (1.0 / del[0]);
-      if (NDIM > 1) dtl = rmax(dtl, (fabs(vy - 0.) + cs) * (1.0 / del[1]));
-      if (NDIM > 2) dtl = rmax(dtl, (fabs(vz - 0.) + cs) * (1.0 / del[2]));
-      CflCand c; c.key = dtl * P.cfl; c.val = dtl; c.idx = loc;
-      cfl_merge(cand, c);
-    }
-  }
-  if (LAST) cfl_block_reduce<NX, NY, NZ>(cand, b, P.cfl, part);
-  if (st) atomicOr(P.status, st);
 }
 
 // CFL reduction of a stored state (Hydro_computeDt on its own).

@@ -11,6 +11,12 @@ namespace fhy {
 // a CTA stages kMxRun blocks that follow one another along the sweep and
 // 1/kMxRun of their cross-section.
 constexpr int kMxRun = 4;
+// The FP64 direction kernels take the same runs with an eighth of the
+// cross-section per CTA (one layer of 8 lines: with 14 doubles of face state
+// per line cell, a quarter would leave one CTA per SM).
+constexpr int kRunParts = 8;
+// CFL candidates kept per block, at most (one per CTA that shares it)
+constexpr int kCflParts = kRunParts;
 
 // Tensor maps of the step's input state for the mixed direction kernels'
 // TMA staging (k_dir_mx, uniform 3D grids): per state variable the block
@@ -32,6 +38,7 @@ struct StepArgs {
   double *aux;        // [ndim-1][3][ncells] eint-update terms of the earlier directions
   size_t ncells;
   CflPart *part;      // per-block CFL results
+  CflCand *cflq = nullptr;  // [nblocks][kCflParts] candidates of the CTAs that share a block (3D)
   int nlaunch;        // CTAs (blocks updated)
   int threads;        // threads per CTA of the transverse-flux and CFL passes
   int dir_threads;    // threads per CTA of the FP64 direction kernels

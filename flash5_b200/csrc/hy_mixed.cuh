@@ -17,59 +17,9 @@
 //    shared reciprocals instead of the reference's repeated divisions).
 #pragma once
 #include "hy_kernels.cuh"
+#include "hy_tma.cuh"
 
 namespace fhy {
-
-// ---------------------------------------------------------------------------
-// TMA staging of the direction kernels' line stencils (uniform 3D grids).
-// Each state variable is described by tensor maps over its natural layout
-// (x fastest, then y, then z of every block: dims 8 x 8 x 8*nblocks); one
-// 3D tile copy brings a block's interior (box 8 x 8 x 8) and one a
-// neighbour's 4-cell slab along the sweep direction (box 4 x 8 x 8,
-// 8 x 4 x 8 or 8 x 8 x 4), straight into the staged layout below.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ unsigned smem_u32(const void *p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-// one bounded poll of phase `parity`; true once it has completed
-__device__ __forceinline__ bool mbar_try(unsigned long long *bar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.b32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// 3D tile copy global -> shared through a tensor map (no multicast)
-// L2 prefetch of [p, p + bytes) as one bulk request (16-byte aligned,
-// bytes a multiple of 16)
-__device__ __forceinline__ void bulk_prefetch_l2(const void *p, unsigned bytes) {
-  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(p), "r"(bytes) : "memory");
-}
-// fetch a tensor map into the descriptor cache ahead of its first copy
-__device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map) {
-  asm volatile("prefetch.tensormap [%0];\n" ::"l"(reinterpret_cast<unsigned long long>(map)) : "memory");
-}
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int c0, int c1, int c2,
-                                            unsigned long long *bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], "
-      "[%2];\n" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<unsigned long long>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
-      : "memory");
-}
-// SM cycles (about a second) a CTA waits for its tile copies before it gives
-// up (FLASH_HY_ERR_TIMEOUT)
-constexpr long long kTmaWaitCycles = 1LL << 31;
 
 // FP64 HLLC (hy_HLLC.F90:94-311) with one division per star state; igm1 =
 // 1/(game - 1) of the cell the face state belongs to.
@@ -125,27 +75,6 @@ __device__ __forceinline__ void hllc_fp64(const DevParams &P, const double *Vm, 
   UC[4] = U[4] * r + (pStar * qStar - p * u) * rden;
 #pragma unroll
   for (int n = 0; n < 5; ++n) Fs[n] = F[n] + S * (UC[n] - U[n]);
-}
-
-// Per block, the K quarter candidates of a run step merged into the block's
-// CFL result, as cfl_block_reduce writes it for a block handled whole
-// (Hydro_computeDt.F90:265-284).
-template <int NX, int NY, int K>
-__global__ void k_cfl_runs(const CflCand *cq, int nblocks, double cfl, CflPart *part) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nblocks) return;
-  CflCand a = cq[(size_t)b * K];
-#pragma unroll
-  for (int q = 1; q < K; ++q) cfl_merge(a, cq[(size_t)b * K + q]);
-  CflPart r;
-  if (a.key > 0.0) {
-    r.dt = cfl / a.val;
-    r.i = a.idx % NX; r.j = (a.idx / NX) % NY; r.k = a.idx / (NX * NY);
-  } else {
-    r.dt = DBL_MAX; r.i = r.j = r.k = -1;
-  }
-  r.blk = b;
-  part[b] = r;
 }
 
 // Lines of a CTA: the block's lines along DIR (K = 1), or, with K > 1, a
@@ -394,19 +323,7 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
     sV[3 * G::SA + q] = V[HVZ]; sV[4 * G::SA + q] = V[HEI];
   }
   if (tma) {
-    // bounded wait for the tile copies; a CTA that gives up flags
-    // FLASH_HY_ERR_TIMEOUT, waits (bounded) once more for its copies in
-    // flight and leaves
-    bool done = false;
-    const long long t0 = clock64();
-    while (!done && clock64() - t0 < kTmaWaitCycles) done = mbar_try(bar, 0);
-    if (__syncthreads_or(!done)) {
-      if (threadIdx.x == 0) atomicOr(P.status, (unsigned)FLASH_HY_ERR_TIMEOUT);
-      const long long t1 = clock64();
-      while (clock64() - t1 < kTmaWaitCycles && !mbar_try(bar, 0)) {
-      }
-      return;
-    }
+    if (!tma_wait(bar, P.status)) return;
     // the copied guard cells' EOS (Eos_getData.F90:80-96 on ENER = eint +
     // ekin, as load_prim); the pressure is not staged (Vs below)
     for (int g = threadIdx.x; g < 8 * G::C; g += NT) {
@@ -896,7 +813,7 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
   }
   __syncthreads();
   if (K == 1 && P.freg) {         // AMR: fine/coarse faces
-    flux_register<NDIM, NX, NY, NZ, DIR>(P, b, bc, sF, G::SC, [](int along, int t1, int t2) {
+    flux_register<NDIM, NX, NY, NZ, DIR>(P, b, bc, 0, sF, G::SC, [](int along, int t1, int t2) {
       return G::at(along, t1 + (DIR == 1 ? NY : NX) * t2, G::LC, 1);
     });
     __syncthreads();
@@ -914,23 +831,11 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
 
   } else {
     // replay: the stored fluxes and pressure sums
-    using FS = FluxStore<NDIM, NX, NY, NZ>;
-    const double *src = FS::base(P, b, DIR);
-    for (int q = threadIdx.x; q < NFLX * FS::NF; q += NT) {
-      const int v = q / FS::NF, f = q % FS::NF;
-      int a, t1, t2;
-      face_coords<NDIM, NX, NY, NZ, DIR>(f, a, t1, t2);
-      sF[v * G::SC + fidx(a, t1, t2)] = src[q];
-    }
-    for (int c = threadIdx.x; c < FS::NCB; c += NT) {
-      const int i = c % NX, j = (c / NX) % NY, k = c / (NX * NY);
-      sF[8 * G::SC + fidx(DIR == 1 ? i : (DIR == 2 ? j : k), DIR == 1 ? j : i, DIR == 3 ? j : k)] =
-          src[NFLX * FS::NF + c];
-    }
+    flux_load<NDIM, NX, NY, NZ, DIR>(P, b, 0, sF, G::SC, fidx, [&](int t, double sp) { sF[8 * G::SC + t] = sp; });
     __syncthreads();
   }
   if (K == 1 && (P.fmode == 1 || P.fmode == 2)) {
-    flux_store<NDIM, NX, NY, NZ, DIR>(P, b, sF, G::SC, fidx, [&](int t) { return sF[8 * G::SC + t]; });
+    flux_store<NDIM, NX, NY, NZ, DIR>(P, b, 0, sF, G::SC, fidx, [&](int t) { return sF[8 * G::SC + t]; });
     if (P.fmode == 2) {
       if (st) atomicOr(P.status, st);
       return;
@@ -1036,34 +941,10 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
     if constexpr (K == 1) {
       cfl_block_reduce<NX, NY, NZ>(cand[0], b, P.cfl, part);
     } else {
-      // the CTA's candidate for each block of the run; k_cfl_runs merges
-      // the K quarters of every block (the same max / first-index rule, so
-      // the result equals a reduction over the whole block)
-      // (one barrier: every warp reduces its K candidates, then thread m
-      // merges the warps' candidates of block m)
-      __shared__ CflCand red[32][K];
-      const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-      for (int m = 0; m < K; ++m) {
-        CflCand c = cand[m];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          CflCand o2;
-          o2.key = __shfl_down_sync(0xffffffffu, c.key, o);
-          o2.val = __shfl_down_sync(0xffffffffu, c.val, o);
-          o2.idx = __shfl_down_sync(0xffffffffu, c.idx, o);
-          if (lane + o < 32) cfl_merge(c, o2);
-        }
-        if (lane == 0) red[w][m] = c;
-      }
-      __syncthreads();
-      if (threadIdx.x < K) {
-        const int m = threadIdx.x;
-        CflCand a = red[0][m];
-        for (int q = 1; q < NT / 32; ++q) cfl_merge(a, red[q][m]);
-        const int bm = tm.runs[(size_t)(blockIdx.x / K) * (K + 2) + m];   // blk[m] (not indexed at run time)
-        static_cast<CflCand *>(tm.cflq)[(size_t)bm * K + qtr] = a;
-      }
+      // (the same max / first-index rule as a reduction over the whole block)
+      cfl_parts_reduce<K>(cand, [&](int bm) {
+        return static_cast<CflCand *>(tm.cflq) + (size_t)tm.runs[(size_t)(blockIdx.x / K) * (K + 2) + bm] * K + qtr;
+      });
     }
   }
   if (st) atomicOr(P.status, st);

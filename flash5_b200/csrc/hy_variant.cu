@@ -11,6 +11,8 @@
 #include "../../include/flash_hy.h"
 #if FHY_VARIANT == 3
 #include "hy_mixed.cuh"
+#else
+#include "hy_dir64.cuh"
 #endif
 
 #if FHY_VARIANT == 3
@@ -31,10 +33,10 @@ typedef double Real;
 
 namespace fhy {
 
-// the mixed direction kernels take runs of kMxRun blocks (full uniform 3D
-// grids with run maps, the plain step)
+// the direction kernels take runs of blocks (full uniform 3D grids with run
+// maps, the plain step)
 static bool use_runs(const StepArgs &a) {
-  return FHY_VARIANT == 3 && a.tma_run && a.nlev == 0 && a.P.blk_list == nullptr && a.P.fmode == 0 &&
+  return a.tma_run && a.nlev == 0 && a.P.blk_list == nullptr && a.P.fmode == 0 &&
          a.nlaunch == a.nblocks;
 }
 
@@ -47,16 +49,9 @@ static bool launch_dir_one(const StepArgs &a) {
   constexpr int NT = MxThreads<NDIM, NX, NY, NZ>::pick(FHY_MXSEL);
   auto kern = k_dir_mx<NDIM, NX, NY, NZ, DIR, FIRST, LAST, RS, NT, 1, ORD>;
   const int threads = NT;
-#else
-  static_assert(ORD == 0, "the FP64 variants sweep x, y, z");
-  using G = DirGeom<NDIM, NX, NY, NZ, Real, DIR>;
-  auto kern = k_dir<NDIM, NX, NY, NZ, Real, DIR, FIRST, LAST, FHY_VARIANT, RS>;
-  const int threads = a.dir_threads;
-#endif
   const size_t smem = G::smem_bytes();
   if (a.set_attr && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return false;
-#if FHY_VARIANT == 3
   TmaLine tl;
   memset(&tl, 0, sizeof tl);
   if constexpr (NDIM == 3) {
@@ -70,15 +65,40 @@ static bool launch_dir_one(const StepArgs &a) {
       tl = a.tma_run[DIR - 1];
       kr<<<a.nlaunch, threads, smr, a.stream>>>(a.P, (const Real *)a.sig, a.acc, a.aux, a.ncells, a.part, tl);
       if (LAST)
-        k_cfl_runs<NX, NY, kMxRun><<<(a.nblocks + 255) / 256, 256, 0, a.stream>>>(
-            static_cast<const CflCand *>(tl.cflq), a.nblocks, a.P.cfl, a.part);
+        k_cfl_merge<NX, NY, kMxRun><<<(a.nblocks + 255) / 256, 256, 0, a.stream>>>(a.cflq, nullptr, a.nblocks, a.P.cfl,
+                                                                                   a.part);
       return cudaGetLastError() == cudaSuccess;
     }
   }
   if (NDIM == 3 && a.tma && a.nlev == 0) tl = a.tma[DIR - 1];
   kern<<<a.nlaunch, threads, smem, a.stream>>>(a.P, (const Real *)a.sig, a.acc, a.aux, a.ncells, a.part, tl);
 #else
-  kern<<<a.nlaunch, threads, smem, a.stream>>>(a.P, (const Real *)a.sig, a.acc, a.aux, a.ncells, a.part);
+  static_assert(ORD == 0, "the FP64 variants sweep x, y, z");
+  TmaLine tl;
+  memset(&tl, 0, sizeof tl);
+  if constexpr (NDIM == 3) {
+    if (use_runs(a)) {
+      using G = Dir64<NDIM, NX, NY, NZ, DIR, kRunParts, kMxRun>;
+      auto kern = k_dir<NDIM, NX, NY, NZ, DIR, FIRST, LAST, FHY_VARIANT, RS, kRunParts, kMxRun>;
+      const size_t smem = G::smem_bytes();
+      if (a.set_attr && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        return false;
+      // one pass of every phase at 288 threads (288 slope cells, 272 line cells)
+      constexpr int most = Dir64Bounds<NDIM, NX, kMxRun>::threads;
+      const int threads = a.dir_threads < most ? a.dir_threads : most;
+      kern<<<a.nlaunch / kMxRun * kRunParts, threads, smem, a.stream>>>(a.P, (const Real *)a.sig, a.acc, a.aux,
+                                                                       a.ncells, a.part, a.cflq, a.tma_run[DIR - 1]);
+      return cudaGetLastError() == cudaSuccess;
+    }
+  }
+  constexpr int Q = dir64_parts<NDIM>();
+  using G = Dir64<NDIM, NX, NY, NZ, DIR, Q, 1>;
+  auto kern = k_dir<NDIM, NX, NY, NZ, DIR, FIRST, LAST, FHY_VARIANT, RS, Q, 1>;
+  const size_t smem = G::smem_bytes();
+  if (a.set_attr && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    return false;
+  const int threads = a.dir_threads;
+  kern<<<a.nlaunch * Q, threads, smem, a.stream>>>(a.P, (const Real *)a.sig, a.acc, a.aux, a.ncells, a.part, a.cflq, tl);
 #endif
   return cudaGetLastError() == cudaSuccess;
 }
@@ -87,15 +107,29 @@ static bool launch_dir_one(const StepArgs &a) {
 // level, finest first
 template <int NDIM, int NX, int NY, int NZ, int DIR, bool FIRST, bool LAST, int RS, int ORD = 0>
 static bool launch_dir(const StepArgs &a) {
-  if (a.nlev == 0) return launch_dir_one<NDIM, NX, NY, NZ, DIR, FIRST, LAST, RS, ORD>(a);
-  StepArgs b = a;
-  for (int l = a.nlev; l >= 1; --l) {
-    if (a.lev_count[l] == 0) continue;
-    b.P.blk_list = a.lev_list[l];
-    b.nlaunch = a.lev_count[l];
-    if (!launch_dir_one<NDIM, NX, NY, NZ, DIR, FIRST, LAST, RS, ORD>(b)) return false;
-    b.set_attr = false;
+  if (a.nlev == 0) {
+    if (!launch_dir_one<NDIM, NX, NY, NZ, DIR, FIRST, LAST, RS, ORD>(a)) return false;
+  } else {
+    StepArgs b = a;
+    for (int l = a.nlev; l >= 1; --l) {
+      if (a.lev_count[l] == 0) continue;
+      b.P.blk_list = a.lev_list[l];
+      b.nlaunch = a.lev_count[l];
+      if (!launch_dir_one<NDIM, NX, NY, NZ, DIR, FIRST, LAST, RS, ORD>(b)) return false;
+      b.set_attr = false;
+    }
   }
+#if FHY_VARIANT != 3
+  // the CTAs that share a block left a CFL candidate each
+  constexpr int Q = dir64_parts<NDIM>();
+  if (LAST && Q > 1 && a.P.fmode != 2) {
+    const int *list = a.nlev ? a.leaves : a.P.blk_list;
+    const int n = a.nlev ? a.nleaves : a.nlaunch;
+    if (use_runs(a)) k_cfl_merge<NX, NY, kRunParts><<<(n + 255) / 256, 256, 0, a.stream>>>(a.cflq, list, n, a.P.cfl, a.part);
+    else k_cfl_merge<NX, NY, Q><<<(n + 255) / 256, 256, 0, a.stream>>>(a.cflq, list, n, a.P.cfl, a.part);
+    return cudaGetLastError() == cudaSuccess;
+  }
+#endif
   return true;
 }
 
@@ -165,7 +199,9 @@ static int run_rs(const StepArgs &a) {
     ok = launch_dir<NDIM, NX, NY, NZ, 1, true, false, RS>(a) &&
          launch_dir<NDIM, NX, NY, NZ, 2, false, false, RS>(a) &&
          launch_dir<NDIM, NX, NY, NZ, 3, false, true, RS>(a);
-    return ok ? nsig + 3 * nl + (use_runs(a) ? 1 : 0) : -2;   // + the CFL merge of the runs
+    // + the CFL merge of the runs / of the parts of the FP64 kernel's blocks
+    const bool merge = FHY_VARIANT == 3 ? use_runs(a) : a.P.fmode != 2;
+    return ok ? nsig + 3 * nl + (merge ? 1 : 0) : -2;
   }
 }
 

@@ -294,7 +294,7 @@ __device__ __forceinline__ void spec_dir(const DevParams &P, int b, int3 bc, int
   else spec_faces<NDIM, NX, NY, NZ, DIR>(P, slot, sV, sX, sF, sK);
   __syncthreads();
   if (P.sp_freg) {
-    flux_register_v<NDIM, NX, NY, NZ, DIR>(P, b, bc, sF, 0, [](int along, int t1, int t2) {
+    flux_register_v<NDIM, NX, NY, NZ, DIR>(P, b, bc, 0, sF, 0, [](int along, int t1, int t2) {
       const int i = DIR == 1 ? along : t1, j = DIR == 1 ? t1 : (DIR == 2 ? along : t2),
                 k = DIR == 3 ? along : (NDIM > 2 ? t2 : 0);
       return L::idx(i, j, k);

@@ -1,4 +1,7 @@
-"""The division used by the FP64 species pass (``div_rn`` in
+"""The divisions of the FP64 kernels (flash5_b200/csrc/hy_core.cuh): the
+branch-free one of the direction kernels (``Arith<true>``, Newton's
+iteration from a 20-bit seed, restated here with a truncated seed) and the
+division used by the FP64 species pass (``div_rn`` in
 flash5_b200/csrc/hy_core.cuh): x / b from rb = RN(1 / b) with one FMA
 correction (Markstein's theorem).  Restated here in C and compared bit for
 bit with IEEE division on random operands (constants 3 and 6 of the PPM
@@ -31,6 +34,27 @@ static void check(double x, double b) {
   double q = div_rn(x, b, 1. / b), r = x / b;
   if (memcmp(&q, &r, 8) && !(isnan(q) && isnan(r))) { if (bad < 5) printf("x=%a b=%a q=%a r=%a\n", x, b, q, r); ++bad; }
 }
+/* Arith<true>: the seed keeps 20 bits of the reciprocal of b's leading 32 */
+static double seed(double b) { uint64_t u; memcpy(&u, &b, 8); u &= 0xFFFFFFFF00000000ull; memcpy(&b, &u, 8);
+  double y = 1. / b; memcpy(&u, &y, 8); u &= 0xFFFFFFFF00000000ull; memcpy(&y, &u, 8); return y; }
+static int in_rng(double x) { uint64_t u; memcpy(&u, &x, 8); return ((uint32_t)(u >> 32) & 0x7fffffffu) - 0x20B00000u < 0x3E800000u; }
+static int refused(double x, double b) {
+  uint64_t u, v; memcpy(&u, &b, 8); memcpy(&v, &x, 8);
+  const uint32_t hi = (uint32_t)(u >> 32);
+  const int ones = ((hi | 0xfff00000u) & (uint32_t)u) == 0xffffffffu;
+  return !in_rng(b) || ones || (!in_rng(x) && ((uint32_t)(v >> 32) & 0x7fffffffu) != 0);
+}
+static double div_bf(double x, double b) {
+  double y = seed(b);
+  const double e = fma(-b, y, 1.);
+  y = fma(y, fma(e, e, e), y);
+  const double r = fma(y, fma(-b, y, 1.), y), q0 = x * r;
+  return fma(-fma(q0, b, -x), r, q0);
+}
+static void checkf(double x, double b) {
+  double q = div_bf(x, b), r = x / b;
+  if (!refused(x, b) && memcmp(&q, &r, 8)) { if (bad < 5) printf("x=%a b=%a q=%a r=%a\n", x, b, q, r); ++bad; }
+}
 int main(void) {
   const double cs[] = {3., 6.};
   for (int c = 0; c < 2; ++c)
@@ -42,6 +66,21 @@ int main(void) {
   }
   const double sp[] = {0., -0., 1e-310, -1e-310, 5e-324, 1e308, -1e308, INFINITY, -INFINITY, NAN};
   for (int i = 0; i < 10; ++i) { check(sp[i], 3.); check(sp[i], 6.); check(sp[i], 1e-3); check(sp[i], 7.5e9); }
+  long b0 = bad;
+  for (long i = 0; i < 12000000; ++i) {
+    const double x = i % 3 ? rnd(-60, 60) : rnd(-499, 499);
+    double b = fabs(i % 5 ? rnd(-40, 40) : rnd(-499, 499));
+    if (i % 7 == 0) { uint64_t bb; memcpy(&bb, &b, 8); bb |= 0xFFFFFFFFFFFF0ull; memcpy(&b, &bb, 8); }
+    checkf(x, b);
+  }
+  for (long i = 0; i < 3000000; ++i) { checkf(rnd(-60, 60), 3.); checkf(rnd(-60, 60), 6.); checkf(rnd(-60, 60), 12.); }
+  const double z[] = {0., -0.};
+  for (int i = 0; i < 2; ++i) { checkf(z[i], 3.); checkf(z[i], 0.7); }
+  const double out[] = {1e-310, 1e200, INFINITY, NAN, -1e-160};
+  for (int i = 0; i < 5; ++i) if (!refused(out[i], 1.5)) { printf("not refused %g\n", out[i]); ++bad; }
+  { uint64_t ones = 0x3FFFFFFFFFFFFFFFull; double b; memcpy(&b, &ones, 8); if (!refused(1., b)) ++bad; }
+  if (!refused(1., 0.) || !refused(1., 1e300)) ++bad;
+  printf("branch-free: mismatches %ld\n", bad - b0);
   printf("mismatches %ld\n", bad);
   return bad != 0;
 }
