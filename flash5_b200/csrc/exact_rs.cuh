@@ -41,20 +41,53 @@ struct MlpPacked {
 static_assert(sizeof(MlpPacked) % 16 == 0, "MlpPacked must be a multiple of 16 bytes");
 
 // ---------------------------------------------------------------------------
+// reciprocals and roots without branches: Newton's iteration (third order)
+// from the 20-bit seeds of rcp / rsqrt.approx.ftz.f64, the square root with
+// one residual correction.  Within an ulp for operands in [2^-500, 2^500)
+// (the seeds flush subnormals); the compiler's divisions and roots end their
+// basic block with a call for special operands, which keeps a solve's ten of
+// them from overlapping.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ double rcp_nr(double b) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(b));
+  const double e = fma(-b, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double div_nr(double x, double b) {
+  const double y = rcp_nr(b), q = x * y;
+  return fma(fma(-q, b, x), y, q);
+}
+__device__ __forceinline__ double rsqrt_nr(double a) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(a));
+  const double e = fma(-(a * y), y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+__device__ __forceinline__ double sqrt_nr(double a) {
+  const double y = rsqrt_nr(a), q = a * y;
+  return fma(0.5 * y, fma(-q, q, a), q);
+}
+// whether x > 0 lies in [2^-300, 2^300): operands in that range keep the
+// above in theirs
+__device__ __forceinline__ bool in_range(double x) { return (unsigned)__double2hiint(x) - 0x2D300000u < 0x25800000u; }
+
+// ---------------------------------------------------------------------------
 // pressure functions, guess, Newton, star velocity
 //
-// Newton runs on w = p^z, z = (g-1)/(2g), not on p.  In w the rarefaction
-// branch of f_K (Toro eq. 4.7) is linear, f_K = 2 c_K/(g-1) (w/w_K - 1), so
-// the two-rarefaction guess (eq. 4.46) is the root of the linear part and
-// the exact root where both waves are rarefactions.  For g <= 5/3 the
-// shock branch (eq. 4.6) is convex in w, so Newton from the two-rarefaction
-// guess, which lies at or right of the root, descends monotonically; for
-// stiffer gases it is not convex near w_K and the bracket safeguards carry
-// the iteration.  p = w^(1/z) with 1/z = 2 + 2/(g-1) is an integer power
-// for g = 5/3, 7/5, 4/3, so the iteration needs no transcendental function
-// there; w_K = p_K^z is taken once per side.
+// Newton runs on w = (p / p_L)^z, z = (g-1)/(2g), not on p.  In w the
+// rarefaction branch of f_K (Toro eq. 4.7) is linear, f_K = 2 c_K/(g-1)
+// (w/w_K - 1), so the two-rarefaction guess (eq. 4.46) is the root of the
+// linear part and the exact root where both waves are rarefactions.  For g
+// <= 5/3 the shock branch (eq. 4.6) is convex in w, so Newton from the
+// two-rarefaction guess, which lies at or right of the root, descends
+// monotonically; for stiffer gases it is not convex near w_K and the bracket
+// safeguards carry the iteration.  p / p_L = w^(1/z) with 1/z = 2 + 2/(g-1)
+// is an integer power for g = 5/3, 7/5, 4/3, so the iteration needs no
+// transcendental function there; with the pressures taken relative to p_L,
+// w_L = 1 and only w_R = (p_R / p_L)^z is a power, one per solve.
 // ---------------------------------------------------------------------------
-struct Side { double d, u, p, c, w; };              // w = p^z
+struct Side { double d, u, p, c, w; };              // w = (p / p_L)^z: 1 on the left
 
 // x^y for x > 0 as exp2(y log2 x): the relative error is a few ulp times
 // |y log2 x|, far below the solver's tolerance, at a fraction of the cost
@@ -79,28 +112,31 @@ __device__ __forceinline__ double pow_k(double x, double k) {
 
 __host__ __device__ __forceinline__ double zexp(double g) { return (g - 1.0) / (2.0 * g); }
 
-// p = w^n, n = 1/z = 2g/(g-1): unrolled for the integer exponents of
-// g = 5/3, 7/5, 4/3 (5, 7, 8), else pow_k
+// P = w^n, n = 1/z = 2g/(g-1): unrolled for the integer exponents of
+// g = 5/3, 7/5, 4/3 (5, 7, 8; the same instructions with a selected factor,
+// so that lanes of different gases do not diverge), else pow_k
 struct PowN { int ni; double n; };
-__host__ __device__ __forceinline__ PowN pown_of(double g) {
-  const double n = 2.0 * g / (g - 1.0), r = rint(n);
+__host__ __device__ __forceinline__ PowN pown_of(double n) {
+  const double r = rint(n);
   return PowN{(fabs(n - r) < 1e-9 && (r == 5.0 || r == 7.0 || r == 8.0)) ? (int)r : 0, n};
 }
 __device__ __forceinline__ double pow_n(double w, const PowN &e) {
-  if (e.ni == 5) { const double w2 = w * w; return w2 * w2 * w; }
-  if (e.ni == 7) { const double w2 = w * w, w4 = w2 * w2; return w4 * w2 * w; }
-  if (e.ni == 8) { const double w2 = w * w, w4 = w2 * w2; return w4 * w4; }
-  return pow_k(w, e.n);
+  if (e.ni == 0) return pow_k(w, e.n);
+  const double w2 = w * w, w4 = w2 * w2;
+  return w4 * (e.ni == 5 ? w : (e.ni == 7 ? w2 * w : w4));
 }
-// p = w^n and dp/dw = n w^(n-1), the latter from the same powers for the
+// P = w^n and dP/dw = n w^(n-1), the latter from the same powers for the
 // integer exponents (no division)
 __device__ __forceinline__ double pow_n_d(double w, const PowN &e, double &dpdw) {
-  if (e.ni == 5) { const double w2 = w * w, w4 = w2 * w2; dpdw = 5.0 * w4; return w4 * w; }
-  if (e.ni == 7) { const double w2 = w * w, w6 = w2 * w2 * w2; dpdw = 7.0 * w6; return w6 * w; }
-  if (e.ni == 8) { const double w2 = w * w, w4 = w2 * w2, w7 = w4 * w2 * w; dpdw = 8.0 * w7; return w7 * w; }
-  const double p = pow_k(w, e.n);
-  dpdw = e.n * p / w;
-  return p;
+  if (e.ni == 0) {
+    const double p = pow_k(w, e.n);
+    dpdw = e.n * p / w;
+    return p;
+  }
+  const double w2 = w * w, w3 = w2 * w, w4 = w2 * w2;
+  const double m = e.ni == 5 ? 1.0 : (e.ni == 7 ? w2 : w3), q = w4 * m;     // w^(n-1)
+  dpdw = e.n * q;
+  return q * w;
 }
 
 // Constants of the gas, taken once per context on the host where the
@@ -110,6 +146,7 @@ __device__ __forceinline__ double pow_n_d(double w, const PowN &e, double &dpdw)
 // two-rarefaction guess and the sampling (section 4.5).
 struct Gas {
   double g, z, gm1inv, k2, a2, g6, g2, hgm1;   // 1/(g-1), 2/(g-1), 2/(g+1), (g-1)/(g+1), (g+1)/(2g), (g-1)/2
+  double s0;                                   // sqrt(2/((g+1) g)): sqrt(A_K p_K) = s0 c_K
   PowN e;
 };
 __host__ __device__ __forceinline__ Gas gas_of(double g) {
@@ -122,47 +159,71 @@ __host__ __device__ __forceinline__ Gas gas_of(double g) {
   s.g6 = (g - 1.0) / (g + 1.0);
   s.g2 = (g + 1.0) / (2.0 * g);
   s.hgm1 = 0.5 * (g - 1.0);
-  s.e = pown_of(g);
+  s.s0 = sqrt(s.a2 / g);
+  s.e = pown_of(2.0 * g / (g - 1.0));
+  return s;
+}
+// the same without branches, for a gas per solve
+__device__ __forceinline__ Gas gas_nr(double g) {
+  Gas s;
+  const double gm1 = g - 1.0, r1 = rcp_nr(gm1), r2 = rcp_nr(g + 1.0);
+  s.g = g;
+  s.z = div_nr(gm1, 2.0 * g);
+  s.gm1inv = r1;
+  s.k2 = 2.0 * r1;
+  s.a2 = 2.0 * r2;
+  s.g6 = gm1 * r2;
+  s.g2 = 1.0 - s.z;
+  s.hgm1 = 0.5 * gm1;
+  s.s0 = sqrt_nr(div_nr(s.a2, g));
+  s.e = pown_of(2.0 * g * r1);
   return s;
 }
 
+// p / p_L of w
 __device__ __forceinline__ double p_of_w(double w, const Gas &G) { return pow_n(w, G.e); }
-__device__ __forceinline__ Side make_side(double d, double u, double p, double c, const Gas &G) {
-  return Side{d, u, p, c, powp(p, G.z)};
-}
 
-// Constants of one side's pressure function, taken once per solve: w_K,
-// p_K, the rarefaction slope k = 2 c_K / ((g-1) w_K) and A_K, B_K of the
-// shock branch.
-struct SideK { double w, p, k, A, B; };
-__device__ __forceinline__ SideK side_k(const Side &s, const Gas &G) {
-  return SideK{s.w, s.p, G.k2 * s.c / s.w, G.a2 / s.d, G.g6 * s.p};
-}
-
-// f_K(w) and df_K/dw (Toro eqs. 4.6-4.7 with p = w^n, dp/dw = dpdw)
-__device__ __forceinline__ void pres_fn(double w, double p, double dpdw, const SideK &s, double &f, double &fd) {
-  if (w <= s.w) {                                   // rarefaction, Toro eq. 4.7
-    f = s.k * (w - s.w);
-    fd = s.k;
-  } else {                                          // shock, Toro eq. 4.6
-    const double r = 1.0 / (s.B + p);
-    const double q = sqrt(s.A * r);
-    f = (p - s.p) * q;
-    fd = (1.0 - 0.5 * (p - s.p) * r) * q * dpdw;    // df/dp dp/dw
+// One side's pressure function, in pressures relative to p_L: w_K, P_K =
+// p_K / p_L, the rarefaction slope k = 2 c_K / ((g-1) w_K), s = sqrt(A_K
+// p_L) and B_K / p_L of the shock branch.
+struct SideK { double w, P, k, s, B; };
+// sound speeds of a pair (d, u, p given); the branch-free roots hold over
+// [2^-300, 2^300), others take the compiler's
+__device__ __forceinline__ bool sound(Side &L, Side &R, const Gas &G) {
+  const bool fast = in_range(L.d) && in_range(L.p) && in_range(R.d) && in_range(R.p);
+  if (fast) {
+    L.c = sqrt_nr(G.g * L.p * rcp_nr(L.d));
+    R.c = sqrt_nr(G.g * R.p * rcp_nr(R.d));
+  } else {
+    L.c = sqrt(G.g * L.p / L.d);
+    R.c = sqrt(G.g * R.p / R.d);
   }
+  return fast;
+}
+// and w and the pressure functions
+__device__ __forceinline__ void setup(Side &L, Side &R, const Gas &G, SideK &kl, SideK &kr) {
+  const bool fast = sound(L, R, G);
+  const double x = fast ? div_nr(R.p, L.p) : R.p / L.p;
+  L.w = 1.0;
+  R.w = powp(x, G.z);
+  kl = SideK{1.0, 1.0, G.k2 * L.c, G.s0 * L.c, G.g6};
+  kr = SideK{R.w, x, G.k2 * R.c * rcp_nr(R.w), G.s0 * R.c * rsqrt_nr(x), G.g6 * x};
+}
+
+// f_K(w) and df_K/dw (Toro eqs. 4.6-4.7 with P = w^n, dP/dw = dpdw): both
+// branches, then a select (the shock's square root is one Newton iteration)
+__device__ __forceinline__ void pres_fn(double w, double P, double dpdw, const SideK &s, double &f, double &fd) {
+  const double y = rsqrt_nr(s.B + P), q = s.s * y, dP = P - s.P;
+  const bool shock = w > s.w;
+  f = shock ? dP * q : s.k * (w - s.w);
+  fd = shock ? (1.0 - 0.5 * dP * (y * y)) * q * dpdw : s.k;
 }
 
 // two-rarefaction guess in w (0 where the states generate vacuum), Toro
 // eq. 4.46 with c_K/w_K = k_K (g-1)/2 from the sides' rarefaction slopes
 __device__ __forceinline__ double tr_w(const Side &L, const Side &R, const SideK &kl, const SideK &kr, const Gas &G) {
   const double num = L.c + R.c - G.hgm1 * (R.u - L.u);
-  return num > 0.0 ? num / (G.hgm1 * (kl.k + kr.k)) : 0.0;
-}
-__device__ __forceinline__ double tr_w(const Side &L, const Side &R, const Gas &G) {
-  return tr_w(L, R, side_k(L, G), side_k(R, G), G);
-}
-__device__ __forceinline__ double tr_guess(const Side &L, const Side &R, const Gas &G) {
-  return p_of_w(tr_w(L, R, G), G);
+  return num > 0.0 ? div_nr(num, G.hgm1 * (kl.k + kr.k)) : 0.0;
 }
 
 // vacuum generation test, Toro eq. 4.40
@@ -206,8 +267,8 @@ __device__ __forceinline__ bool strong_screen(double dl, double ul, double pl, d
   return ppv + E > pmin * (1.f - 1e-5f) && fmaxf(pmax * (1.f + 1e-5f), ppv + E) >= 2.f * pmin * (1.f - 1e-5f);
 }
 
-// The star state of a solve: p*, u* and w* = p*^z (the sampling takes the
-// rarefaction-side powers (p*/p_K)^z = w*/w_K from it).
+// The star state of a solve: p*, u* and w* = (p*/p_L)^z (the sampling takes
+// the rarefaction-side powers (p*/p_K)^z = w*/w_K from it).
 struct Star { double p, u, w; };
 
 // Newton on f(w) = f_L + f_R + (u_R - u_L) from w0 >= 0.  Converged when
@@ -225,41 +286,28 @@ __device__ __forceinline__ int newton(const Side &L, const Side &R, const SideK 
   const double du = R.u - L.u, ztol = G.z * tol;
   const PowN &e = G.e;
   double wa = 0.0, wb = DBL_MAX;
-  double w = w0, prev = -1.0, p = 0.0;
-  double fl = 0., fdl = 0., fr = 0., fdr = 0., we = w0;
+  double w = w0, prev = -1.0;
+  double fl = 0., fdl = 0., fr = 0., fdr = 0., we = w0, wend = w0;
   int evals = 0;
-  for (; evals < max_iter;) {
+  bool done = false;
+  while (evals < max_iter && !done) {
     double dpdw;
-    p = pow_n_d(w, e, dpdw);
-    pres_fn(w, p, dpdw, kl, fl, fdl);
-    pres_fn(w, p, dpdw, kr, fr, fdr);
+    const double P = pow_n_d(w, e, dpdw);
+    pres_fn(w, P, dpdw, kl, fl, fdl);
+    pres_fn(w, P, dpdw, kr, fr, fdr);
     ++evals;
     we = w;
     const double f = fl + fr + du;
-    if (f == 0.0) {
-      out.w = w; out.p = p;
-      out.u = 0.5 * (L.u + R.u) + 0.5 * (fr - fl);
-      return evals;
-    }
-    if (f < 0.0) wa = w; else wb = w;
-    if (wb - wa <= ztol * w) {
-      out.w = 0.5 * (wa + wb);
-      out.p = pow_n(out.w, e);
-      const double dw = out.w - we;
-      out.u = 0.5 * (L.u + R.u) + 0.5 * ((fr + fdr * dw) - (fl + fdl * dw));
-      return evals;
-    }
-    const double step = f / (fdl + fdr);
+    if (f < 0.0) wa = w;
+    else if (f > 0.0) wb = w;
+    const double step = f * rcp_nr(fdl + fdr);
     double wn = w - step;
     const double as = fabs(step);
-    const bool inside = wn > wa && wn < wb;
-    if (as <= ztol * w || (inside && prev > 0.0 && as < prev && as * (as / prev) * (as / prev) <= 0.01 * ztol * w)) {
-      out.w = wn > 0.0 ? wn : w;
-      out.p = pow_n(out.w, e);
-      const double dw = out.w - we;
-      out.u = 0.5 * (L.u + R.u) + 0.5 * ((fr + fdr * dw) - (fl + fdl * dw));
-      return evals;
-    }
+    const bool narrow = wb - wa <= ztol * w, inside = wn > wa && wn < wb;
+    // f == 0: the root; a narrow bracket: its midpoint; else the step
+    done = f == 0.0 || narrow || as <= ztol * w ||
+           (inside && prev > 0.0 && as < prev && as * as * as <= 0.01 * ztol * w * (prev * prev));
+    wend = f == 0.0 ? w : (narrow ? 0.5 * (wa + wb) : (wn > 0.0 ? wn : w));
     if (!inside) {
       wn = wb == DBL_MAX ? 2.0 * w : 0.5 * (wa + wb);
       prev = -1.0;
@@ -268,78 +316,58 @@ __device__ __forceinline__ int newton(const Side &L, const Side &R, const SideK 
     }
     w = wn;
   }
-  out.w = w; out.p = pow_n(w, e);
-  const double dw = w - we;
+  if (!done) wend = w;
+  const double dw = wend - we;
+  out.w = wend;
+  out.p = L.p * pow_n(wend, e);
   out.u = 0.5 * (L.u + R.u) + 0.5 * ((fr + fdr * dw) - (fl + fdl * dw));
-  return -max_iter;
+  return done ? evals : -max_iter;
 }
 
 // ---------------------------------------------------------------------------
 // the exact solution at x/t = 0 (Toro 4.5; vacuum generation 4.6)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void fan_left(const Side &L, const Gas &G, double &d, double &u, double &p) {
-  const double c = G.a2 * (L.c + G.hgm1 * L.u);
+// inside the fan of side K, velocities mirrored so that K lies on the left
+__device__ __forceinline__ void fan(const Side &K, double uk, const Gas &G, double &d, double &u, double &p) {
+  const double c = G.a2 * (K.c + G.hgm1 * uk);
   u = c;
-  const double r = c / L.c;
-  d = L.d * pow_k(r, G.k2);
-  p = L.p * pow_n(r, G.e);
-}
-__device__ __forceinline__ void fan_right(const Side &R, const Gas &G, double &d, double &u, double &p) {
-  const double c = G.a2 * (R.c - G.hgm1 * R.u);
-  u = -c;
-  const double r = c / R.c;
-  d = R.d * pow_k(r, G.k2);
-  p = R.p * pow_n(r, G.e);
+  const double r = c / K.c;
+  d = K.d * pow_k(r, G.k2);
+  p = K.p * pow_n(r, G.e);
 }
 
-// (d, u, p) at x/t = 0 and which side supplies the transverse velocities;
-// behind a rarefaction (p*/p_K)^z = w*/w_K and rho*_K = rho_K (w*/w_K)^(2/(g-1))
+// (d, u, p) at x/t = 0 and which side supplies the transverse velocities.
+// The side of the contact that holds x/t = 0 is mirrored onto the left, so
+// one copy of the wave tests serves both; behind a rarefaction (p*/p_K)^z =
+// w*/w_K and rho*_K = rho_K (w*/w_K)^(2/(g-1)).
 __device__ __forceinline__ void sample0(const Side &L, const Side &R, const Gas &G, const Star &S, bool vac,
                                         double &d, double &u, double &p, bool &right) {
   if (vac) {
     const double sl = L.u + G.k2 * L.c, sr = R.u - G.k2 * R.c;
     if (0.0 <= L.u - L.c) { right = false; d = L.d; u = L.u; p = L.p; }
-    else if (0.0 < sl) { right = false; fan_left(L, G, d, u, p); }
+    else if (0.0 < sl) { right = false; fan(L, L.u, G, d, u, p); }
     else if (0.0 >= R.u + R.c) { right = true; d = R.d; u = R.u; p = R.p; }
-    else if (0.0 > sr) { right = true; fan_right(R, G, d, u, p); }
+    else if (0.0 > sr) { right = true; fan(R, -R.u, G, d, u, p); u = -u; }
     else { right = false; d = 0.0; u = 0.0; p = 0.0; }
     return;
   }
-  const double ps = S.p, us = S.u;
-  const double g1 = G.z, g2 = G.g2, g6 = G.g6, k = G.k2;
-  if (0.0 <= us) {                                   // left of the contact
-    right = false;
-    if (ps > L.p) {                                  // left shock
-      const double pr = ps / L.p;
-      const double sl = L.u - L.c * sqrt(g2 * pr + g1);
-      if (0.0 <= sl) { d = L.d; u = L.u; p = L.p; }
-      else { d = L.d * (pr + g6) / (pr * g6 + 1.0); u = us; p = ps; }
-    } else {                                         // left rarefaction
-      if (0.0 <= L.u - L.c) { d = L.d; u = L.u; p = L.p; }
-      else {
-        const double q = S.w / L.w;
-        const double cml = L.c * q;
-        if (0.0 > us - cml) { d = L.d * pow_k(q, k); u = us; p = ps; }
-        else fan_left(L, G, d, u, p);
-      }
-    }
-  } else {                                           // right of the contact
-    right = true;
-    if (ps > R.p) {
-      const double pr = ps / R.p;
-      const double sr = R.u + R.c * sqrt(g2 * pr + g1);
-      if (0.0 >= sr) { d = R.d; u = R.u; p = R.p; }
-      else { d = R.d * (pr + g6) / (pr * g6 + 1.0); u = us; p = ps; }
-    } else {
-      if (0.0 >= R.u + R.c) { d = R.d; u = R.u; p = R.p; }
-      else {
-        const double q = S.w / R.w;
-        const double cmr = R.c * q;
-        if (0.0 <= us + cmr) { d = R.d * pow_k(q, k); u = us; p = ps; }
-        else fan_right(R, G, d, u, p);
-      }
-    }
+  right = !(0.0 <= S.u);
+  Side K;
+  K.d = right ? R.d : L.d; K.u = right ? -R.u : L.u; K.p = right ? R.p : L.p; K.c = right ? R.c : L.c;
+  K.w = right ? R.w : L.w;
+  const double ps = S.p, us = right ? -S.u : S.u;
+  if (ps > K.p) {                                  // shock
+    const double pr = div_nr(ps, K.p);
+    if (0.0 <= K.u - K.c * sqrt_nr(G.g2 * pr + G.z)) { d = K.d; u = K.u; p = K.p; }
+    else { d = K.d * div_nr(pr + G.g6, pr * G.g6 + 1.0); u = us; p = ps; }
+  } else if (0.0 <= K.u - K.c) {                   // rarefaction
+    d = K.d; u = K.u; p = K.p;
+  } else {
+    const double q = div_nr(S.w, K.w);
+    if (0.0 >= us - K.c * q) { d = K.d * pow_k(q, G.k2); u = us; p = ps; }
+    else fan(K, K.u, G, d, u, p);
   }
+  if (right) u = -u;
 }
 
 // Godunov flux of the exact solution in the 6-slot layout of the HLLC

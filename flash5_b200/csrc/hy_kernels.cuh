@@ -444,10 +444,11 @@ __global__ void k_cfl_merge(const CflCand *cq, const int *list, int n, double cf
 // ---------------------------------------------------------------------------
 // exact Riemann face flux (no FLASH5 counterpart; Toro ch. 4, exact_rs.cuh)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ xrs::Side side_of(const double *V, int n, const xrs::Gas &G, unsigned &st) {
-  const double c2 = G.g * V[HP] / V[HD];
-  if (!(c2 > 0.0)) st |= ST_NEG_SOUND;
-  return xrs::make_side(V[HD], V[n], V[HP], sqrt(c2), G);
+// a side's density, normal velocity and pressure; a squared sound speed that
+// is not positive is reported
+__device__ __forceinline__ xrs::Side side_of(double d, double u, double p, unsigned &st) {
+  if (!((p > 0.0 && d > 0.0) || (p < 0.0 && d < 0.0))) st |= ST_NEG_SOUND;
+  return xrs::Side{d, u, p, 0.0, 0.0};
 }
 
 // keep a hashed sample of the face states (two-rarefaction guess inexact) for
@@ -469,13 +470,12 @@ __device__ __forceinline__ void harvest_face(const DevParams &P, const xrs::Side
 template <int DIR>
 __device__ __forceinline__ void exact_face(const DevParams &P, const xrs::Gas &G, const double *VL, const double *VR,
                                            double F[6], unsigned &st) {
-  const xrs::Side L = side_of(VL, DIR, G, st), R = side_of(VR, DIR, G, st);
+  xrs::Side L = side_of(VL[HD], VL[DIR], VL[HP], st), R = side_of(VR[HD], VR[DIR], VR[HP], st);
+  xrs::SideK kl, kr;
+  xrs::setup(L, R, G, kl, kr);
   const bool vac = xrs::vacuum(L, R, G);
   xrs::Star S{0.0, 0.5 * (L.u + R.u), 0.0};
-  if (!vac) {
-    const xrs::SideK kl = xrs::side_k(L, G), kr = xrs::side_k(R, G);
-    if (xrs::newton(L, R, kl, kr, G, xrs::tr_w(L, R, kl, kr, G), P.rs_tol, P.rs_max_iter, S) < 0) st |= ST_NEWTON;
-  }
+  if (!vac && xrs::newton(L, R, kl, kr, G, xrs::tr_w(L, R, kl, kr, G), P.rs_tol, P.rs_max_iter, S) < 0) st |= ST_NEWTON;
   xrs::godunov_flux<DIR>(VL, VR, L, R, G, S, vac, F);
 }
 

@@ -628,19 +628,10 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
       return left ? Vs(qq, s.y) + double(sWp[qq * G::SC + t - G::step])
                   : Vs(qq, s.x) + double(sWm[qq * G::SC + t]);
     };
-    // the two face states; w = p^z only with `with_w` (pass 1a tests for
-    // strong waves without it)
-    auto sides = [&](int2 s, int t, xrs::Side &L, xrs::Side &R, bool with_w = true) {
-      const double dl = face(0, true, s, t), ul = face(DIR, true, s, t), pl = face(4, true, s, t);
-      const double dr = face(0, false, s, t), ur = face(DIR, false, s, t), pr = face(4, false, s, t);
-      const double c2l = g * pl / dl, c2r = g * pr / dr;
-      if (!(c2l > 0.0) || !(c2r > 0.0)) st |= ST_NEG_SOUND;
-      L = xrs::Side{dl, ul, pl, sqrt(c2l), 0.0};
-      R = xrs::Side{dr, ur, pr, sqrt(c2r), 0.0};
-      if (with_w) {
-        L.w = xrs::powp(pl, gas.z);
-        R.w = xrs::powp(pr, gas.z);
-      }
+    // the two face states (sound speeds and the rest by xrs::sound / setup)
+    auto sides = [&](int2 s, int t, xrs::Side &L, xrs::Side &R) {
+      L = side_of(face(0, true, s, t), face(DIR, true, s, t), face(4, true, s, t), st);
+      R = side_of(face(0, false, s, t), face(DIR, false, s, t), face(4, false, s, t), st);
     };
     if (learned) {
       // pass 1a: faces with strong waves and an inexact two-rarefaction
@@ -659,12 +650,13 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
         if (xrs::strong_screen(face(0, true, s4, t), face(DIR, true, s4, t), face(4, true, s4, t),
                                face(0, false, s4, t), face(DIR, false, s4, t), face(4, false, s4, t), g)) {
           xrs::Side L, R;
-          sides(s4, t, L, R, false);
+          sides(s4, t, L, R);
+          xrs::sound(L, R, gas);
           if (!xrs::vacuum(L, R, gas) && xrs::strong_waves(L, R)) {
-            L.w = xrs::powp(L.p, gas.z);
-            R.w = xrs::powp(R.p, gas.z);
-            const double wtr = xrs::tr_w(L, R, gas);
-            if (!xrs::tr_exact(L, R, xrs::p_of_w(wtr, gas))) q = wtr;
+            xrs::SideK kl, kr;
+            xrs::setup(L, R, gas, kl, kr);
+            const double wtr = xrs::tr_w(L, R, kl, kr, gas);
+            if (!xrs::tr_exact(L, R, L.p * xrs::p_of_w(wtr, gas))) q = wtr;
           }
         }
         sP0[t] = q;
@@ -686,9 +678,12 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
           const bool net = q > 0.0;
           if (!__any_sync(0xffffffffu, net)) continue;
           xrs::Side L{1.0, 0.0, 1.0, 1.0, 1.0}, R{1.0, 0.0, 1.0, 1.0, 1.0};
-          if (net) sides(make_int2(G::sidx(x, l), G::sidx(x - 1, l)), t, L, R);
+          if (net) {
+            sides(make_int2(G::sidx(x, l), G::sidx(x - 1, l)), t, L, R);
+            xrs::sound(L, R, gas);
+          }
           float f[xrs::NIN];
-          if (net) xrs::features(L, R, g, xrs::p_of_w(q, gas), f);
+          if (net) xrs::features(L, R, g, L.p * xrs::p_of_w(q, gas), f);
           else {
 #pragma unroll
             for (int k = 0; k < xrs::NIN; ++k) f[k] = 0.f;
@@ -711,12 +706,13 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
       if (x < 0) continue;
       const int2 s = make_int2(G::sidx(x, l), G::sidx(x - 1, l));
       xrs::Side L, R;
+      xrs::SideK kl, kr;
       sides(s, t, L, R);
+      xrs::setup(L, R, gas, kl, kr);
       const bool vac = xrs::vacuum(L, R, gas);
       xrs::Star S{0.0, 0.5 * (L.u + R.u), 0.0};
       if (!vac) {
         const double q = learned ? sP0[t] : 0.0;
-        const xrs::SideK kl = xrs::side_k(L, gas), kr = xrs::side_k(R, gas);
         const double w0 = q < 0.0 ? -q : xrs::tr_w(L, R, kl, kr, gas);
         // the network's start gets three evaluations; if they do not
         // converge, Newton restarts from the two-rarefaction guess
@@ -729,7 +725,7 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
           if (k >= 0 || !net) break;
         }
         if (k < 0) st |= ST_NEWTON;
-        if (P.harvest && (q < 0.0 || (xrs::strong_waves(L, R) && !xrs::tr_exact(L, R, xrs::p_of_w(w0, gas)))))
+        if (P.harvest && (q < 0.0 || (xrs::strong_waves(L, R) && !xrs::tr_exact(L, R, L.p * xrs::p_of_w(w0, gas)))))
           harvest_face(P, L, R, g, (unsigned)(blockIdx.x * 4 + DIR) * 2048u + (unsigned)t);
       }
       double VL[8], VR[8];

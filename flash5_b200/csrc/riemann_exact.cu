@@ -37,25 +37,19 @@ using namespace xrs;
 // ---------------------------------------------------------------------------
 constexpr int SOLVE_THREADS = 256;
 
-__device__ __forceinline__ void load_state(const double *__restrict__ S, long n, long i, Side &L, Side &R, Gas &G) {
+__device__ __forceinline__ void load_state(const double *__restrict__ S, long n, long i, Side &L, Side &R, Gas &G,
+                                           SideK &kl, SideK &kr) {
   L.d = S[i]; L.u = S[n + i]; L.p = S[2 * n + i];
   R.d = S[3 * n + i]; R.u = S[4 * n + i]; R.p = S[5 * n + i];
-  const double g = S[6 * n + i];
-  G = gas_of(g);
-  L.c = sqrt(g * L.p / L.d); R.c = sqrt(g * R.p / R.d);
-  L.w = powp(L.p, G.z); R.w = powp(R.p, G.z);
+  G = gas_nr(S[6 * n + i]);
+  setup(L, R, G, kl, kr);
 }
 
-// the state of pair i, or a harmless placeholder for a lane past the end
+// the state of pair i, or that of the last pair for a lane past the end
 // (lanes of the last tile take part in the warp and CTA collectives)
-__device__ __forceinline__ void load_or_dummy(const double *__restrict__ S, long n, long i, bool valid, Side &L,
-                                              Side &R, Gas &G) {
-  if (valid) {
-    load_state(S, n, i, L, R, G);
-  } else {
-    G = gas_of(1.4);
-    L.d = R.d = 1.0; L.u = R.u = 0.0; L.p = R.p = 1.0; L.c = R.c = sqrt(1.4); L.w = R.w = 1.0;
-  }
+__device__ __forceinline__ void load_or_last(const double *__restrict__ S, long n, long i, Side &L, Side &R, Gas &G,
+                                             SideK &kl, SideK &kr) {
+  load_state(S, n, i < n ? i : n - 1, L, R, G, kl, kr);
 }
 
 // Newton from w0 (three evaluations where the network gave the start, else
@@ -106,9 +100,12 @@ __device__ __forceinline__ void enqueue(bool pending, long i, int *queue, int *q
 // warp waits for a fallback lane.  Here the network runs per warp on
 // mma.sync (mlp_lane); k_solve_tc below is the tcgen05 form.
 // One instantiation per path, so that the two-rarefaction path does not
-// carry the network's register footprint.
+// carry the network's register footprint.  Bound by FP64 issue and latency;
+// 1e8 pairs on B200, two-rarefaction start: 8.84 ms with two powers, IEEE
+// divisions and roots per solve (16 warps per SM) -> 4.33 ms with one power
+// and branch-free arithmetic (exact_rs.cuh), 4.24 at 64 registers (32 warps).
 template <bool learned>
-__global__ void __launch_bounds__(SOLVE_THREADS, learned ? 2 : 1)
+__global__ void __launch_bounds__(SOLVE_THREADS, learned ? 2 : 4)
 k_solve(const double *__restrict__ S, long n, double *__restrict__ out, unsigned char *__restrict__ iters,
         unsigned char *__restrict__ flags, const MlpPacked *__restrict__ w, double tol, int max_iter, int *queue,
         int *qcount, unsigned *status) {
@@ -122,11 +119,11 @@ k_solve(const double *__restrict__ S, long n, double *__restrict__ out, unsigned
     const bool valid = i < n;
     Side L, R;
     Gas G;
-    load_or_dummy(S, n, i, valid, L, R, G);
-    const SideK kl = side_k(L, G), kr = side_k(R, G);
+    SideK kl, kr;
+    load_or_last(S, n, i, L, R, G, kl, kr);
     const bool vac = vacuum(L, R, G);
     const double wtr = vac ? 0.0 : tr_w(L, R, kl, kr, G);
-    const double ptr = vac ? 0.0 : p_of_w(wtr, G);
+    const double ptr = vac ? 0.0 : L.p * p_of_w(wtr, G);
     double w0 = wtr;
     bool net = false;
     if (learned) {
@@ -202,8 +199,8 @@ __device__ __forceinline__ uint32_t relu_bf16x2(float lo, float hi) {
 }
 
 // Five CTAs per SM for the solve (96 registers, a few spilled), six for
-// the network alone (80): measured on 1e8 pairs, 11.1 -> 10.5 ms and
-// 5.6 -> 5.4 ms against four.
+// the network alone (80): measured on 1e8 pairs, solve 7.6 ms against 8.3 at
+// six and seven; network 5.4 ms against 5.6 at four.
 template <bool SOLVE>
 __global__ void __launch_bounds__(TC_THREADS, SOLVE ? 5 : 6)
 k_solve_tc(const double *__restrict__ S, long n, double *__restrict__ out, unsigned char *__restrict__ iters,
@@ -268,11 +265,11 @@ k_solve_tc(const double *__restrict__ S, long n, double *__restrict__ out, unsig
     const bool valid = i < n;
     Side L, R;
     Gas G;
-    load_or_dummy(S, n, i, valid, L, R, G);
-    const SideK kl = side_k(L, G), kr = side_k(R, G);
+    SideK kl, kr;
+    load_or_last(S, n, i, L, R, G, kl, kr);
     const bool vac = vacuum(L, R, G);
     const double wtr = vac ? 0.0 : tr_w(L, R, kl, kr, G);
-    const double ptr = vac ? 0.0 : p_of_w(wtr, G);
+    const double ptr = vac ? 0.0 : L.p * p_of_w(wtr, G);
     const bool net = SOLVE ? (valid && !vac && !tr_exact(L, R, ptr) && strong_waves(L, R)) : (valid && !vac);
     float y = 0.f;
     {
@@ -397,10 +394,10 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_fallback(const double *__rest
     const long i = queue[q];
     Side L, R;
     Gas G;
-    load_state(S, n, i, L, R, G);
+    SideK kl, kr;
+    load_state(S, n, i, L, R, G, kl, kr);
     Star S;
     unsigned char fl = 1 | 8;
-    const SideK kl = side_k(L, G), kr = side_k(R, G);
     int k = newton(L, R, kl, kr, G, tr_w(L, R, kl, kr, G), tol, max_iter, S);
     int its = 3 + (k > 0 ? k : max_iter);
     if (k <= 0) { fl |= 4; st |= FLASH_HY_ERR_NEWTON_NOCONV; }
@@ -425,9 +422,10 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_predict(const double *__restr
     if (i < n) {
       Side L, R;
       Gas G;
-      load_state(S, n, i, L, R, G);
+      SideK kl, kr;
+      load_state(S, n, i, L, R, G, kl, kr);
       vac = vacuum(L, R, G);
-      if (!vac) features(L, R, G.g, tr_guess(L, R, G), f);
+      if (!vac) features(L, R, G.g, L.p * p_of_w(tr_w(L, R, kl, kr, G), G), f);
     }
     const float yy = mlp_lane(M, f);
     if (i < n) y[i] = vac ? 0.f : yy;
@@ -470,11 +468,12 @@ __global__ void k_make_samples(const double *S, const double *out, long n, float
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     Side L, R;
     Gas G;
-    load_state(S, n, i, L, R, G);
+    SideK kl, kr;
+    load_state(S, n, i, L, R, G, kl, kr);
     if (vacuum(L, R, G)) continue;
     double ps = out[i];
     if (!(ps > 0.0)) continue;
-    double ptr = tr_guess(L, R, G);
+    double ptr = L.p * p_of_w(tr_w(L, R, kl, kr, G), G);
     if (tr_exact(L, R, ptr) || !strong_waves(L, R)) continue;   // where the network is consulted
     int k = atomicAdd(count, 1);
     if (k >= cap) continue;
