@@ -211,19 +211,21 @@ __device__ __forceinline__ void setup(Side &L, Side &R, const Gas &G, SideK &kl,
 }
 
 // f_K(w) and df_K/dw (Toro eqs. 4.6-4.7 with P = w^n, dP/dw = dpdw): both
-// branches, then a select (the shock's square root is one Newton iteration)
+// branches, then a select (the shock's square root is one Newton iteration).
+// Here and below sums of products are spelled out (fma, __dmul_rn), so that
+// every kernel that inlines the solver rounds alike.
 __device__ __forceinline__ void pres_fn(double w, double P, double dpdw, const SideK &s, double &f, double &fd) {
-  const double y = rsqrt_nr(s.B + P), q = s.s * y, dP = P - s.P;
+  const double y = rsqrt_nr(__dadd_rn(s.B, P)), q = __dmul_rn(s.s, y), dP = __dsub_rn(P, s.P);
   const bool shock = w > s.w;
-  f = shock ? dP * q : s.k * (w - s.w);
-  fd = shock ? (1.0 - 0.5 * dP * (y * y)) * q * dpdw : s.k;
+  f = shock ? __dmul_rn(dP, q) : __dmul_rn(s.k, w - s.w);
+  fd = shock ? fma(-0.5 * dP, __dmul_rn(y, y), 1.0) * q * dpdw : s.k;
 }
 
 // two-rarefaction guess in w (0 where the states generate vacuum), Toro
 // eq. 4.46 with c_K/w_K = k_K (g-1)/2 from the sides' rarefaction slopes
 __device__ __forceinline__ double tr_w(const Side &L, const Side &R, const SideK &kl, const SideK &kr, const Gas &G) {
-  const double num = L.c + R.c - G.hgm1 * (R.u - L.u);
-  return num > 0.0 ? div_nr(num, G.hgm1 * (kl.k + kr.k)) : 0.0;
+  const double num = fma(-G.hgm1, R.u - L.u, L.c + R.c);
+  return num > 0.0 ? div_nr(num, G.hgm1 * __dadd_rn(kl.k, kr.k)) : 0.0;
 }
 
 // vacuum generation test, Toro eq. 4.40
@@ -297,10 +299,10 @@ __device__ __forceinline__ int newton(const Side &L, const Side &R, const SideK 
     pres_fn(w, P, dpdw, kr, fr, fdr);
     ++evals;
     we = w;
-    const double f = fl + fr + du;
+    const double f = __dadd_rn(fl, fr) + du;
     if (f < 0.0) wa = w;
     else if (f > 0.0) wb = w;
-    const double step = f * rcp_nr(fdl + fdr);
+    const double step = __dmul_rn(f, rcp_nr(__dadd_rn(fdl, fdr)));
     double wn = w - step;
     const double as = fabs(step);
     const bool narrow = wb - wa <= ztol * w, inside = wn > wa && wn < wb;
@@ -320,7 +322,7 @@ __device__ __forceinline__ int newton(const Side &L, const Side &R, const SideK 
   const double dw = wend - we;
   out.w = wend;
   out.p = L.p * pow_n(wend, e);
-  out.u = 0.5 * (L.u + R.u) + 0.5 * ((fr + fdr * dw) - (fl + fdl * dw));
+  out.u = 0.5 * (L.u + R.u) + 0.5 * (fma(fdr, dw, fr) - fma(fdl, dw, fl));
   return done ? evals : -max_iter;
 }
 
@@ -329,7 +331,7 @@ __device__ __forceinline__ int newton(const Side &L, const Side &R, const SideK 
 // ---------------------------------------------------------------------------
 // inside the fan of side K, velocities mirrored so that K lies on the left
 __device__ __forceinline__ void fan(const Side &K, double uk, const Gas &G, double &d, double &u, double &p) {
-  const double c = G.a2 * (K.c + G.hgm1 * uk);
+  const double c = G.a2 * fma(G.hgm1, uk, K.c);
   u = c;
   const double r = c / K.c;
   d = K.d * pow_k(r, G.k2);
@@ -358,13 +360,13 @@ __device__ __forceinline__ void sample0(const Side &L, const Side &R, const Gas 
   const double ps = S.p, us = right ? -S.u : S.u;
   if (ps > K.p) {                                  // shock
     const double pr = div_nr(ps, K.p);
-    if (0.0 <= K.u - K.c * sqrt_nr(G.g2 * pr + G.z)) { d = K.d; u = K.u; p = K.p; }
-    else { d = K.d * div_nr(pr + G.g6, pr * G.g6 + 1.0); u = us; p = ps; }
+    if (0.0 <= fma(-K.c, sqrt_nr(fma(G.g2, pr, G.z)), K.u)) { d = K.d; u = K.u; p = K.p; }
+    else { d = K.d * div_nr(pr + G.g6, fma(pr, G.g6, 1.0)); u = us; p = ps; }
   } else if (0.0 <= K.u - K.c) {                   // rarefaction
     d = K.d; u = K.u; p = K.p;
   } else {
     const double q = div_nr(S.w, K.w);
-    if (0.0 >= us - K.c * q) { d = K.d * pow_k(q, G.k2); u = us; p = ps; }
+    if (0.0 >= fma(-K.c, q, us)) { d = K.d * pow_k(q, G.k2); u = us; p = ps; }
     else fan(K, K.u, G, d, u, p);
   }
   if (right) u = -u;
@@ -383,10 +385,10 @@ __device__ __forceinline__ void godunov_flux(const double *VL, const double *VR,
   double v[3];
 #pragma unroll
   for (int m = 0; m < 3; ++m) v[m] = (m == DIR - 1) ? u : (right ? VR[1 + m] : VL[1 + m]);
-  const double E = p * G.gm1inv + 0.5 * d * (v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-  F[0] = d * u;
+  const double E = fma(0.5 * d, fma(v[0], v[0], fma(v[1], v[1], __dmul_rn(v[2], v[2]))), __dmul_rn(p, G.gm1inv));
+  F[0] = __dmul_rn(d, u);
   F[1] = F[0] * v[0]; F[2] = F[0] * v[1]; F[3] = F[0] * v[2];
-  F[DIR] += p;
+  F[DIR] = fma(F[0], u, p);
   F[4] = (E + p) * u;
   F[5] = p;
 }

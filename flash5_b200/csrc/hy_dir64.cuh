@@ -307,14 +307,6 @@ __device__ __forceinline__ void hllc64(const DevParams &P, A &ar, const double *
 // slots stored for the face states: dens, velx, vely, velz, pres, eint
 __device__ __forceinline__ int wslot(int q) { return q < 5 ? q : HEI; }
 
-// blk[m] without indexing registers at run time
-template <int K> __device__ __forceinline__ int pick(const int (&blk)[K], int m) {
-  int b = blk[0];
-#pragma unroll
-  for (int q = 1; q < K; ++q) b = m == q ? blk[q] : b;
-  return b;
-}
-
 template <int NDIM, int NX, int NY, int NZ, int DIR, bool FIRST, bool LAST, int VAR, int RS, int Q, int K>
 __global__ void __launch_bounds__(Dir64Bounds<NDIM, NX, K>::threads, Dir64Bounds<NDIM, NX, K>::ctas)
 k_dir(const DevParams P, const double *__restrict__ SIG, double *__restrict__ ACC, double *__restrict__ AUX,

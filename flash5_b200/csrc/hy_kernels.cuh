@@ -353,6 +353,14 @@ __device__ __forceinline__ void load_sig(const double *p, size_t stride, double 
   s[HGC] = 0.; s[HGE] = 0.;
 }
 
+// blk[m] without indexing registers at run time
+template <int K> __device__ __forceinline__ int pick(const int (&blk)[K], int m) {
+  int b = blk[0];
+#pragma unroll
+  for (int q = 1; q < K; ++q) b = m == q ? blk[q] : b;
+  return b;
+}
+
 // deterministic (max key, first index) reduction for the CFL step
 struct CflCand { double key, val; int idx; };
 __device__ __forceinline__ void cfl_merge(CflCand &a, const CflCand &b) {

@@ -8,27 +8,31 @@
 namespace fhy {
 
 // Blocks per run of the mixed direction kernels on full uniform 3D grids:
-// a CTA stages kMxRun blocks that follow one another along the sweep and
-// 1/kMxRun of their cross-section.
+// a CTA stages kMxRun blocks that follow one another along the sweep and a
+// part of their cross-section.
 constexpr int kMxRun = 4;
-// The FP64 direction kernels take the same runs with an eighth of the
-// cross-section per CTA (one layer of 8 lines: with 14 doubles of face state
-// per line cell, a quarter would leave one CTA per SM).
-constexpr int kRunParts = 8;
+// Parts of the cross-section a run CTA takes.  An eighth (one layer of 8
+// lines; 288 threads pass every phase once, three CTAs per SM): the mixed
+// HLLC kernels (KH 160^3 step 1.64 ms against 1.71 on quarters at 320
+// threads, two CTAs) and the FP64 kernels (with 14 doubles of face state per
+// line cell a quarter leaves one CTA per SM).  A quarter: the mixed
+// exact-solver kernels, whose face solve spills at an eighth's 72 registers
+// (KH 256^3 8.16 against 8.45 ms).
+__host__ __device__ constexpr int run_parts(bool mixed, bool exact) { return mixed && exact ? 4 : 8; }
 // CFL candidates kept per block, at most (one per CTA that shares it)
-constexpr int kCflParts = kRunParts;
+constexpr int kCflParts = 8;
 
 // Tensor maps of the step's input state for the mixed direction kernels'
 // TMA staging (k_dir_mx, uniform 3D grids): per state variable the block
 // interior (box 8 x 8 x 8) and the neighbour slab along the sweep direction
 // (box 4 x 8 x 8, 8 x 4 x 8 or 8 x 8 x 4) over the natural block layout;
-// for runs, the same boxes cut to 1/kMxRun of the slower transverse axis.
+// for runs, the same boxes cut to one part of the slower transverse axis.
 struct TmaLine {
   CUtensorMap intr[5];        // dens, velx, vely, velz, eint
   CUtensorMap slab[5];
   int on;                     // 0: the stencil is staged by load_prim
   const int *runs;            // runs: [nblocks / kMxRun][kMxRun + 2] blocks along the sweep, neighbours below / above
-  void *cflq;                 // runs, last direction: [nblocks][kMxRun] CflCand of the quarters
+  void *cflq;                 // runs, last direction: [nblocks][parts] CflCand of the parts
 };
 
 struct StepArgs {

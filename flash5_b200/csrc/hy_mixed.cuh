@@ -21,60 +21,92 @@
 
 namespace fhy {
 
-// FP64 HLLC (hy_HLLC.F90:94-311) with one division per star state; igm1 =
-// 1/(game - 1) of the cell the face state belongs to.
+// whether x lies in [lo, 2^300), lo a positive double given by its high word
+__device__ __forceinline__ bool at_least(double x, int lo) { return __double2hiint(x) - lo > 0 && __double2hiint(x) < 0x52B00000; }
+
+// FP64 HLLC (hy_HLLC.F90:94-311) and the volume flux F_dens / rho of the
+// upwind side; ig = 1/(game - 1), that of the gamma law.  Branch-free: one
+// reciprocal per density and per star state (xrs::rcp_nr), both sides' tests
+// by selects.  Densities and pressures that vanish, are negative or leave
+// the range of the branch-free arithmetic take hllc_any.  Sums of products
+// are spelled out (fma, __dmul_rn), so that every compiled candidate of the
+// kernel rounds alike.
 template <int DIR>
-__device__ __forceinline__ void hllc_fp64(const DevParams &P, const double *Vm, const double *Vp, double igL,
-                                          double igR, double Fs[6], unsigned &st) {
+__device__ __forceinline__ void hllc_any(const DevParams &P, const double *Vm, const double *Vp, double ig,
+                                         double Fs[6], double &fv, unsigned &st) {
   constexpr int v1 = Slots<DIR>::v1;
   const double tiny = P.tiny;
-  if ((Vm[HD] < tiny && Vm[HD] > 0.) || (Vp[HD] < tiny && Vp[HD] > 0.) || (Vm[HP] < tiny && Vm[HP] > 0.) ||
-      (Vp[HP] < tiny && Vp[HP] > 0.)) {
-#pragma unroll
-    for (int n = 0; n < 6; ++n) Fs[n] = 0.;
-    return;
-  }
   const double uL = Vm[v1], uR = Vp[v1], dL = Vm[HD], dR = Vp[HD], pL = Vm[HP], pR = Vp[HP];
   const double aL2 = P.gamma * pL / dL, aR2 = P.gamma * pR / dR;
-  if (aL2 < 0. || aR2 < 0.) {
-    st |= ST_NEG_SOUND;
+  const bool vanish = (dL < tiny && dL > 0.) || (dR < tiny && dR > 0.) || (pL < tiny && pL > 0.) || (pR < tiny && pR > 0.);
+  if (vanish || aL2 < 0. || aR2 < 0.) {
+    if (!vanish) st |= ST_NEG_SOUND;
 #pragma unroll
     for (int n = 0; n < 6; ++n) Fs[n] = 0.;
+    fv = 0.;
     return;
   }
   const double cL = sqrt(aL2), cR = sqrt(aR2);
   const double SL = fmin(uL - cL, uR - cR), SR = fmax(uL + cL, uR + cR);
-  double qStar = (dR * uR * (SR - uR) - dL * uL * (SL - uL) + pL - pR) / (dR * (SR - uR) - dL * (SL - uL));
-  // side whose flux (and star state) is used
+  const double qStar = (dR * uR * (SR - uR) - dL * uL * (SL - uL) + pL - pR) / (dR * (SR - uR) - dL * (SL - uL));
   const bool useL = SL >= 0. || qStar >= 0.;
   const double *V = useL ? Vm : Vp;
   const double d = useL ? dL : dR, u = useL ? uL : uR, p = useL ? pL : pR, S = useL ? SL : SR;
-  const double ig = useL ? igL : igR;
-  const double u2 = V[HVX] * V[HVX] + V[HVY] * V[HVY] + V[HVZ] * V[HVZ];
-  const double E = 0.5 * d * u2 + p * ig;
-  double F[5], U[5];
+  const double E = 0.5 * d * (V[HVX] * V[HVX] + V[HVY] * V[HVY] + V[HVZ] * V[HVZ]) + p * ig;
+  double F[5];
   F[0] = d * u;
   F[1] = F[0] * V[HVX]; F[2] = F[0] * V[HVY]; F[3] = F[0] * V[HVZ];
   F[DIR] += p;
   F[4] = (E + p) * u;
   Fs[5] = p;
-  const bool outside = useL ? (SL >= 0.) : (SR < 0.);
-  if (outside) {
+  if (useL ? (SL >= 0.) : (SR < 0.)) {
 #pragma unroll
     for (int n = 0; n < 5; ++n) Fs[n] = F[n];
-    return;
+  } else {
+    const double rden = 1.0 / (S - qStar), r = (S - u) * rden;
+    const double pStar = dL * (SL - uL) * (qStar - uL) + pL;
+    const double U[5] = {d, d * V[HVX], d * V[HVY], d * V[HVZ], E};
+    double UC[5];
+    UC[0] = d * r;
+#pragma unroll
+    for (int m = 1; m <= 3; ++m) UC[m] = (m == DIR) ? UC[0] * qStar : U[m] * r;
+    UC[4] = E * r + (pStar * qStar - p * u) * rden;
+#pragma unroll
+    for (int n = 0; n < 5; ++n) Fs[n] = F[n] + S * (UC[n] - U[n]);
   }
-  U[0] = d; U[1] = d * V[HVX]; U[2] = d * V[HVY]; U[3] = d * V[HVZ]; U[4] = E;
-  const double num = S - u, rden = 1.0 / (S - qStar);
-  const double r = num * rden;
-  const double pStar = dL * (SL - uL) * (qStar - uL) + pL;
-  double UC[5];
-  UC[0] = d * r;
-#pragma unroll
-  for (int m = 1; m <= 3; ++m) UC[m] = (m == DIR) ? UC[0] * qStar : U[m] * r;
-  UC[4] = U[4] * r + (pStar * qStar - p * u) * rden;
-#pragma unroll
-  for (int n = 0; n < 5; ++n) Fs[n] = F[n] + S * (UC[n] - U[n]);
+  fv = Fs[0] / (Fs[0] > 0. ? dL : dR);
+}
+template <int DIR>
+__device__ __forceinline__ bool hllc_fp64(const DevParams &P, const double *Vm, const double *Vp, double ig,
+                                          double Fs[6], double &fv) {
+  constexpr int v1 = Slots<DIR>::v1;
+  const double uL = Vm[v1], uR = Vp[v1], dL = Vm[HD], dR = Vp[HD], pL = Vm[HP], pR = Vp[HP];
+  const int lo = max(__double2hiint(P.tiny), 0x2D300000);          // tiny or 2^-300
+  const bool ok = at_least(dL, lo) && at_least(dR, lo) && at_least(pL, lo) && at_least(pR, lo);
+  const double rL = xrs::rcp_nr(dL), rR = xrs::rcp_nr(dR);
+  const double cL = xrs::sqrt_nr(P.gamma * pL * rL), cR = xrs::sqrt_nr(P.gamma * pR * rR);
+  const double SL = fmin(uL - cL, uR - cR), SR = fmax(uL + cL, uR + cR);
+  const double mL = __dmul_rn(dL, SL - uL), mR = __dmul_rn(dR, SR - uR);
+  const double qStar = (fma(uR, mR, -__dmul_rn(uL, mL)) + (pL - pR)) * xrs::rcp_nr(__dsub_rn(mR, mL));
+  const double pStar = fma(mL, qStar - uL, pL);
+  // side whose flux (and star state) is used
+  const bool useL = SL >= 0. || qStar >= 0.;
+  const double vx = useL ? Vm[HVX] : Vp[HVX], vy = useL ? Vm[HVY] : Vp[HVY], vz = useL ? Vm[HVZ] : Vp[HVZ];
+  const double d = useL ? dL : dR, u = useL ? uL : uR, p = useL ? pL : pR, S = useL ? SL : SR;
+  const double E = fma(0.5 * d, fma(vx, vx, fma(vy, vy, __dmul_rn(vz, vz))), __dmul_rn(p, ig));
+  const bool star = useL ? !(SL >= 0.) : !(SR < 0.);
+  // F + S (U* - U), U* = d r (1, v*, ...) with r - 1 = (q - u) / (S - q); F
+  // alone outside the fan
+  const double rden = xrs::rcp_nr(S - qStar), r1 = __dmul_rn(qStar - u, rden);
+  const double f0 = __dmul_rn(d, u), g = __dmul_rn(S, d), fn = fma(f0, u, p), fe = __dmul_rn(E + p, u);
+  const double a = star ? fma(g, r1, f0) : f0;
+  Fs[0] = a;
+  Fs[1] = a * vx; Fs[2] = a * vy; Fs[3] = a * vz;
+  Fs[DIR] = star ? fma(g, fma(r1, qStar, qStar - u), fn) : fn;
+  Fs[4] = star ? fma(S, fma(E, r1, __dmul_rn(fma(pStar, qStar, -__dmul_rn(p, u)), rden)), fe) : fe;
+  Fs[5] = p;
+  fv = a * (a > 0. ? rL : rR);
+  return ok;
 }
 
 // Lines of a CTA: the block's lines along DIR (K = 1), or, with K > 1, a
@@ -83,14 +115,14 @@ __device__ __forceinline__ void hllc_fp64(const DevParams &P, const double *Vm, 
 // lines are K blocks long, so the stencil overlap along DIR (four guard
 // cells on each side, recomputed slopes and face states at the ends) is
 // paid once per run instead of once per block.
-template <int NDIM, int NX, int NY, int NZ, int DIR, int RS = 0, int K = 1>
+template <int NDIM, int NX, int NY, int NZ, int DIR, int RS = 0, int K = 1, int Q = 1>
 struct MxGeom {
   static constexpr int ND0 = DIR == 1 ? NX : (DIR == 2 ? NY : NZ);               // block extent along DIR
   static constexpr int ND = K * ND0;                                              // line interior
   static constexpr int T1 = DIR == 1 ? NY : NX;                                   // faster transverse axis
   static constexpr int T2 = DIR == 3 ? NY : NZ;                                   // slower one (split by K)
-  static_assert(K == 1 || (NDIM == 3 && T2 % K == 0), "runs split the slower transverse axis");
-  static constexpr int T2Q = T2 / K;
+  static_assert(Q == 1 || (NDIM == 3 && T2 % Q == 0), "runs split the slower transverse axis");
+  static constexpr int T2Q = T2 / Q;
   static constexpr int C = T1 * T2Q;                                              // lines
   static constexpr int L4 = ND + 8, LS = ND + 4, LC = ND + 2;                      // staged, slope, line cells
   static constexpr int SA = L4 * C, SB = LS * C, SC = LC * C;
@@ -139,7 +171,8 @@ struct MxGeom {
   static constexpr size_t slope_bytes = (size_t)SB * 4 + (size_t)SB * 6 * 4;
   static constexpr size_t wp_off =
       (RS == 1 && slope_bytes < sizeof(xrs::MlpPacked)) ? sizeof(xrs::MlpPacked) : slope_bytes;
-  static constexpr size_t recon_bytes = wp_off + (size_t)2 * SC * 6 * 4 + (size_t)SC * 8;
+  // (+ the start values of the learned guess)
+  static constexpr size_t recon_bytes = wp_off + (size_t)2 * SC * 6 * 4 + (RS == 1 ? (size_t)SC * 8 : 0);
   static constexpr size_t flux_bytes = (size_t)SC * 9 * 8;
   // + the CTA's face-state ranges (learned gate, 16 warps x 6 floats), the
   // staging barrier and the slack that aligns the tile destinations to 128
@@ -180,12 +213,19 @@ template <int NDIM, int NX, int NY, int NZ> struct MxThreads {
 template <int NDIM, int ORD>
 __host__ __device__ constexpr int aux_slot(int d) { return ORD == 0 ? d - 1 : NDIM - d; }
 
-template <int NDIM, int NX, int NY, int NZ, int DIR, bool FIRST, bool LAST, int RS, int NT, int K = 1, int ORD = 0>
-__global__ void __launch_bounds__(NT, NDIM == 3 ? 2 : 1)
+// CTAs per SM the registers are cut for.  Runs of an eighth of the
+// cross-section three (27 warps at 72 registers), quarters and one-block 3D
+// CTAs two.  2D: as many as hold 27 warps at 72 registers (a four-quadrant
+// hierarchy's exact-solver step 2.09 ms; two per SM at 96 registers 2.49,
+// four at 56 2.16, one at 116 3.93).
+template <int NDIM, int NT, int Q> constexpr int mx_ctas() { return NDIM == 3 ? (Q == 8 ? 3 : 2) : (27 * 32) / NT; }
+
+template <int NDIM, int NX, int NY, int NZ, int DIR, bool FIRST, bool LAST, int RS, int NT, int K = 1, int Q = 1, int ORD = 0>
+__global__ void __launch_bounds__(NT, mx_ctas<NDIM, NT, Q>())
 k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ ACC, double *__restrict__ AUX,
          size_t ncells, CflPart *part, const __grid_constant__ TmaLine tm) {
   static_assert(NT % 32 == 0, "threads per CTA must be a multiple of 32");
-  using G = MxGeom<NDIM, NX, NY, NZ, DIR, RS, K>;
+  using G = MxGeom<NDIM, NX, NY, NZ, DIR, RS, K, Q>;
   using B = Box<NDIM, NX, NY, NZ>;
   constexpr int NCB = NX * NY * NZ;
   constexpr int NIT = (G::SC + NT - 1) / NT;
@@ -199,7 +239,6 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
   float *sDb = sFlat + G::SB;                                             // [6][SB]
   float *sWp = reinterpret_cast<float *>(reg + G::wp_off);                // [6][SC] increments
   float *sWm = sWp + 6 * G::SC;                                           // [6][SC]
-  double *sIg = reinterpret_cast<double *>(sWm + 6 * G::SC);              // [SC] 1/(game-1)
   double *sF = reinterpret_cast<double *>(reg + G::flux_off);            // [9][SC] face fluxes
 
   static_assert((6 * B::n * 4) % 16 == 0 && (NCB * 8) % 16 == 0, "bulk prefetch sizes must be multiples of 16 bytes");
@@ -212,8 +251,8 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
   if constexpr (K == 1) {
     blk[0] = P.blk_list ? P.blk_list[blockIdx.x] : blockIdx.x;
   } else {
-    const int *run = tm.runs + (size_t)(blockIdx.x / K) * (K + 2);
-    qtr = blockIdx.x % K;
+    const int *run = tm.runs + (size_t)(blockIdx.x / Q) * (K + 2);
+    qtr = blockIdx.x % Q;
 #pragma unroll
     for (int m = 0; m < K; ++m) blk[m] = run[m];
     nbs[0] = run[K];
@@ -234,11 +273,10 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
   // prefetched into L2 at the start, one bulk request per contiguous range
   // (lanes of warp 0), so that the first touch overlaps the staging and the
   // slopes.
-  // (On a run, CTA qtr prefetches the ranges of block qtr of the run: the run's
-  // K CTAs together cover its K blocks.)
-  if (threadIdx.x < 32) {
+  // (On a run, the first K of its CTAs prefetch the ranges of a block each.)
+  if (threadIdx.x < 32 && qtr < K) {
     const int ln = threadIdx.x;
-    const int pb = K == 1 ? b : blk[qtr];
+    const int pb = K == 1 ? b : tm.runs[(size_t)(blockIdx.x / Q) * (K + 2) + qtr];
     const float *ps = K == 1 ? sigb : SIG + (size_t)pb * NDIM * 6 * B::n;
     if (ln < NDIM && ln != DIR - 1 && P.fmode != 3) bulk_prefetch_l2(ps + (size_t)ln * 6 * B::n, 6u * B::n * 4u);
     if (!FIRST && ln >= 4 && ln < 9) bulk_prefetch_l2(ACC + (ln - 4) * ncells + (size_t)pb * NCB, NCB * 8u);
@@ -278,7 +316,7 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
       const int v = o / (K + 2), r = o % (K + 2);
       double *dst = sV + q5[v] * G::SA;
       if (r < K) {
-        tma_load_3d(dst + G::MID + r * G::MIDB, &tm.intr[v], 0, DIR == 3 ? qo : 0, blk[r] * NZ + (DIR == 3 ? 0 : qo),
+        tma_load_3d(dst + G::MID + r * G::MIDB, &tm.intr[v], 0, DIR == 3 ? qo : 0, pick(blk, r) * NZ + (DIR == 3 ? 0 : qo),
                     bar);
       } else if (r == K) {
         // the slab below: the neighbour's last four layers
@@ -317,7 +355,7 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
     G::cell(xl, l, qtr, i, j, k);
     double V[8];
     if constexpr (K == 1) load_prim<NDIM, NX, NY, NZ, false>(P, b, bc, i, j, k, V);
-    else load_prim<NDIM, NX, NY, NZ, false>(P, blk[m], blk_coords(P, blk[m]), i, j, k, V);
+    else load_prim<NDIM, NX, NY, NZ, false>(P, pick(blk, m), blk_coords(P, pick(blk, m)), i, j, k, V);
     const int q = G::sidx(x, l);
     sV[0 * G::SA + q] = V[HD]; sV[1 * G::SA + q] = V[HVX]; sV[2 * G::SA + q] = V[HVY];
     sV[3 * G::SA + q] = V[HVZ]; sV[4 * G::SA + q] = V[HEI];
@@ -390,7 +428,7 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
     G::dec(t, G::LC, 1, x, l);
     const int mb = G::blk_of(x, xl);             // block of the run: its sig box covers xl in [-1, N]
     G::cell(xl, l, qtr, i, j, k);
-    const float *sigc = K == 1 ? sigb : SIG + (size_t)blk[mb] * NDIM * 6 * B::n;
+    const float *sigc = K == 1 ? sigb : SIG + (size_t)pick(blk, mb) * NDIM * 6 * B::n;
     const int s = G::sidx(x, l), sm = G::sidx(x - 1, l), sp = G::sidx(x + 1, l), q = G::at(x, l, G::LS, 2);
     const int qs = G::step;
     float Vc[8], dL[8], dR[8];
@@ -561,8 +599,6 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
       sWp[qq * G::SC + t] = dWp[sl[qq]];
       sWm[qq * G::SC + t] = dWm[sl[qq]];
     }
-    // 1/(game-1) of the cell: game - 1 = p/(e rho) (Eos_putData.F90:105-106)
-    sIg[t] = (Vs(5, s) * rc) / pc;
     if (RS == 1 && P.mlp) {
       const float fp = float(pc), fr = float(rc), fu = float(Vs(v1, s));
       const float q6[6] = {fp + dWm[HP], fp + dWp[HP], fr + dWm[HD], fr + dWp[HD], fu + dWm[v1], fu + dWp[v1]};
@@ -595,11 +631,11 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
     // exact solver.  With a network attached, pass 1 evaluates its
     // tensor-core guess for the faces with strong waves (the network sits
     // over the slope scratch, dead from here on) and leaves the start value
-    // w0 = p0^z in sP0 (over the unused 1/(game-1) array; negative = network
+    // w0 in sP0 (negative = network
     // start, limited to three evaluations; 0 = two-rarefaction start); pass
     // 2 runs Newton and the Godunov flux.  Each thread reads back only its
     // own entries.
-    double *sP0 = sIg;
+    double *sP0 = reinterpret_cast<double *>(sWm + 6 * G::SC);    // [SC]
     // The CTA-wide bound: every face has p_min >= P_lo, p_max <= P_hi and a
     // PVRS estimate ppv <= P_hi + 0.5 (U_hi - U_lo) rho_hi c_hi with c_hi =
     // sqrt(gamma P_hi / rho_lo); strong_waves needs max(p_max, ppv) >= 2
@@ -739,8 +775,10 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
       xrs::godunov_flux<DIR>(VL, VR, L, R, gas, S, vac, F);
       double fv = 0., fe = 0.;
       if (P.use_aux_eint) {
-        if (F[FDENS] > 0.) { fv = F[FDENS] / VL[HD]; fe = F[FDENS] * VL[HEI]; }
-        else { fv = F[FDENS] / VR[HD]; fe = F[FDENS] * VR[HEI]; }
+        const bool up = F[FDENS] > 0.;
+        const double du = up ? VL[HD] : VR[HD];
+        fv = xrs::in_range(du) ? xrs::div_nr(F[FDENS], du) : F[FDENS] / du;
+        fe = F[FDENS] * (up ? VL[HEI] : VR[HEI]);
       }
       F[FEINT] = fe;
       F[FVOLU] = fv;
@@ -758,6 +796,7 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
       }
     }
   } else {
+  const double ig = 1.0 / P.gam1inv;                // game - 1 = p/(e rho) (Eos_putData.F90:105-106)
 #pragma unroll
   for (int it = 0; it < NIT; ++it) {
     const int t = threadIdx.x + it * NT;
@@ -774,13 +813,10 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
       VL[n] = Vs(qq, sL) + double(sWp[qq * G::SC + tl]);
       VR[n] = Vs(qq, s) + double(sWm[qq * G::SC + t]);
     }
-    double F[9];
-    hllc_fp64<DIR>(P, VL, VR, sIg[tl], sIg[t], F, st);
-    double fv = 0., fe = 0.;
-    if (P.use_aux_eint) {
-      if (F[FDENS] > 0.) { fv = F[FDENS] / VL[HD]; fe = F[FDENS] * VL[HEI]; }
-      else { fv = F[FDENS] / VR[HD]; fe = F[FDENS] * VR[HEI]; }
-    }
+    double F[9], fv, fe;
+    if (!hllc_fp64<DIR>(P, VL, VR, ig, F, fv)) hllc_any<DIR>(P, VL, VR, ig, F, fv, st);
+    fe = F[FDENS] * (F[FDENS] > 0. ? VL[HEI] : VR[HEI]);
+    if (!P.use_aux_eint) fv = fe = 0.;
     F[FEINT] = fe;
     F[FVOLU] = fv;
     // N05 + P05 of this cell (n+1/2 pressure sum)
@@ -850,7 +886,7 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
     const int mb = G::blk_of(x, xl);
     G::cell(xl, l, qtr, i, j, k);
     const int loc = (k * NY + j) * NX + i;
-    const size_t off = (size_t)(K == 1 ? b : blk[mb]) * NCB + loc;
+    const size_t off = (size_t)pick(blk, mb) * NCB + loc;
     double FL[NFLX], FR[NFLX];
 #pragma unroll
     for (int n = 0; n < NFLX; ++n) { FL[n] = sF[n * G::SC + t]; FR[n] = sF[n * G::SC + t + G::step]; }
@@ -882,7 +918,7 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
           pb = (0.5 * sx) * 0.5 + sp * 0.25;
         } else {
           const double sy = AUX[5 * ncells + off];
-          pb = (((0.5 * sx) * 0.5 + sy * 0.25) * 4.0 + sp) / 6.0;
+          pb = (((0.5 * sx) * 0.5 + sy * 0.25) * 4.0 + sp) * (1.0 / 6.0);
         }
         IntEner = rho0 * e0 + dt / del[0] * (AUX[off] + pb * AUX[ncells + off]);
         if (NDIM == 2) {
@@ -903,13 +939,14 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
         }
         double pb;
         if (NDIM == 2) pb = (0.5 * ts[0]) * 0.5 + ts[1] * 0.25;
-        else pb = (((0.5 * ts[0]) * 0.5 + ts[1] * 0.25) * 4.0 + ts[2]) / 6.0;
+        else pb = (((0.5 * ts[0]) * 0.5 + ts[1] * 0.25) * 4.0 + ts[2]) * (1.0 / 6.0);
         IntEner = rho0 * e0 + dt / del[0] * (te[0] + pb * tb[0]);
         IntEner += dt / del[1] * (te[1] + pb * tb[1]);
         if (NDIM == 3) IntEner += dt / del[2] * (te[2] + pb * tb[2]);
       }
       double dens = fmax(U[0], P.smlrho);
-      double rinv = 1.0 / dens;
+      const bool fast = xrs::in_range(dens);
+      double rinv = fast ? xrs::rcp_nr(dens) : 1.0 / dens;
       double vx = U[1] * rinv, vy = U[2] * rinv, vz = U[3] * rinv;
       double ener = U[4] * rinv;
       double eaux = IntEner * rinv;
@@ -923,7 +960,8 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
       P.s_out[4][off] = e;
       if (!(isfinite(dens) && isfinite(vx) && isfinite(vy) && isfinite(vz) && isfinite(e))) st |= ST_NAN;
       double pres = dens * e * P.gam1inv;
-      double cs = sqrt(P.gamma * pres * rinv);
+      const double c2 = P.gamma * pres * rinv;
+      double cs = xrs::in_range(c2) ? xrs::sqrt_nr(c2) : sqrt(c2);
       double dtl = (fabs(vx) + cs) * (1.0 / del[0]);
       if (NDIM > 1) dtl = fmax(dtl, (fabs(vy) + cs) * (1.0 / del[1]));
       if (NDIM > 2) dtl = fmax(dtl, (fabs(vz) + cs) * (1.0 / del[2]));
@@ -934,12 +972,12 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
     }
   }
   if constexpr (LAST) {
-    if constexpr (K == 1) {
+    if constexpr (Q == 1) {
       cfl_block_reduce<NX, NY, NZ>(cand[0], b, P.cfl, part);
     } else {
       // (the same max / first-index rule as a reduction over the whole block)
       cfl_parts_reduce<K>(cand, [&](int bm) {
-        return static_cast<CflCand *>(tm.cflq) + (size_t)tm.runs[(size_t)(blockIdx.x / K) * (K + 2) + bm] * K + qtr;
+        return static_cast<CflCand *>(tm.cflq) + (size_t)pick(blk, bm) * Q + qtr;
       });
     }
   }

@@ -47,7 +47,7 @@ static bool launch_dir_one(const StepArgs &a) {
 #if FHY_VARIANT == 3
   using G = MxGeom<NDIM, NX, NY, NZ, DIR, RS>;
   constexpr int NT = MxThreads<NDIM, NX, NY, NZ>::pick(FHY_MXSEL);
-  auto kern = k_dir_mx<NDIM, NX, NY, NZ, DIR, FIRST, LAST, RS, NT, 1, ORD>;
+  auto kern = k_dir_mx<NDIM, NX, NY, NZ, DIR, FIRST, LAST, RS, NT, 1, 1, ORD>;
   const int threads = NT;
   const size_t smem = G::smem_bytes();
   if (a.set_attr && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
@@ -57,15 +57,19 @@ static bool launch_dir_one(const StepArgs &a) {
   if constexpr (NDIM == 3) {
     // full uniform grid: runs of kMxRun blocks along the sweep
     if (use_runs(a)) {
-      using GR = MxGeom<NDIM, NX, NY, NZ, DIR, RS, kMxRun>;
-      auto kr = k_dir_mx<NDIM, NX, NY, NZ, DIR, FIRST, LAST, RS, NT, kMxRun, ORD>;
+      constexpr int Q = run_parts(true, RS == 1);
+      using GR = MxGeom<NDIM, NX, NY, NZ, DIR, RS, kMxRun, Q>;
+      // an eighth's phases have at most 288 cells; the candidates keep their
+      // own thread counts on quarters
+      constexpr int NTR = Q == 8 && NT > 288 ? 288 : NT;
+      auto kr = k_dir_mx<NDIM, NX, NY, NZ, DIR, FIRST, LAST, RS, NTR, kMxRun, Q, ORD>;
       const size_t smr = GR::smem_bytes();
       if (a.set_attr && cudaFuncSetAttribute(kr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smr) != cudaSuccess)
         return false;
       tl = a.tma_run[DIR - 1];
-      kr<<<a.nlaunch, threads, smr, a.stream>>>(a.P, (const Real *)a.sig, a.acc, a.aux, a.ncells, a.part, tl);
+      kr<<<a.nlaunch / kMxRun * Q, NTR, smr, a.stream>>>(a.P, (const Real *)a.sig, a.acc, a.aux, a.ncells, a.part, tl);
       if (LAST)
-        k_cfl_merge<NX, NY, kMxRun><<<(a.nblocks + 255) / 256, 256, 0, a.stream>>>(a.cflq, nullptr, a.nblocks, a.P.cfl,
+        k_cfl_merge<NX, NY, Q><<<(a.nblocks + 255) / 256, 256, 0, a.stream>>>(a.cflq, nullptr, a.nblocks, a.P.cfl,
                                                                                    a.part);
       return cudaGetLastError() == cudaSuccess;
     }
@@ -78,15 +82,16 @@ static bool launch_dir_one(const StepArgs &a) {
   memset(&tl, 0, sizeof tl);
   if constexpr (NDIM == 3) {
     if (use_runs(a)) {
-      using G = Dir64<NDIM, NX, NY, NZ, DIR, kRunParts, kMxRun>;
-      auto kern = k_dir<NDIM, NX, NY, NZ, DIR, FIRST, LAST, FHY_VARIANT, RS, kRunParts, kMxRun>;
+      constexpr int Q = run_parts(false, RS == 1);
+      using G = Dir64<NDIM, NX, NY, NZ, DIR, Q, kMxRun>;
+      auto kern = k_dir<NDIM, NX, NY, NZ, DIR, FIRST, LAST, FHY_VARIANT, RS, Q, kMxRun>;
       const size_t smem = G::smem_bytes();
       if (a.set_attr && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
         return false;
       // one pass of every phase at 288 threads (288 slope cells, 272 line cells)
       constexpr int most = Dir64Bounds<NDIM, NX, kMxRun>::threads;
       const int threads = a.dir_threads < most ? a.dir_threads : most;
-      kern<<<a.nlaunch / kMxRun * kRunParts, threads, smem, a.stream>>>(a.P, (const Real *)a.sig, a.acc, a.aux,
+      kern<<<a.nlaunch / kMxRun * Q, threads, smem, a.stream>>>(a.P, (const Real *)a.sig, a.acc, a.aux,
                                                                        a.ncells, a.part, a.cflq, a.tma_run[DIR - 1]);
       return cudaGetLastError() == cudaSuccess;
     }
@@ -125,7 +130,7 @@ static bool launch_dir(const StepArgs &a) {
   if (LAST && Q > 1 && a.P.fmode != 2) {
     const int *list = a.nlev ? a.leaves : a.P.blk_list;
     const int n = a.nlev ? a.nleaves : a.nlaunch;
-    if (use_runs(a)) k_cfl_merge<NX, NY, kRunParts><<<(n + 255) / 256, 256, 0, a.stream>>>(a.cflq, list, n, a.P.cfl, a.part);
+    if (use_runs(a)) k_cfl_merge<NX, NY, run_parts(false, RS == 1)><<<(n + 255) / 256, 256, 0, a.stream>>>(a.cflq, list, n, a.P.cfl, a.part);
     else k_cfl_merge<NX, NY, Q><<<(n + 255) / 256, 256, 0, a.stream>>>(a.cflq, list, n, a.P.cfl, a.part);
     return cudaGetLastError() == cudaSuccess;
   }
