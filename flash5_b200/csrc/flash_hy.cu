@@ -622,9 +622,9 @@ extern "C" int flash_hy_create(const flash_hy_params *params, const flash_hy_gri
     // runs of the mixed direction kernels: on a full grid whose block
     // counts divide by kMxRun, every block with coordinate = 0 mod kMxRun
     // along the sweep starts a run of kMxRun blocks (+ its neighbours below
-    // and above the run); the species pass keeps one block per CTA
+    // and above the run)
     constexpr int K = fhy::kMxRun;
-    if (c->tma_maps && !partial && c->nsp == 0 && nbx % K == 0 && nby % K == 0 && nbz % K == 0) {
+    if (c->tma_maps && !partial && nbx % K == 0 && nby % K == 0 && nbz % K == 0) {
       bool ok = true;
       for (int d = 0; d < 3 && ok; ++d) {
         std::vector<int> runs;

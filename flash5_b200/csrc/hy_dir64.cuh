@@ -365,6 +365,12 @@ k_dir(const DevParams P, const double *__restrict__ SIG, double *__restrict__ AC
       bulk_prefetch_l2(AUX + (ln - 12) * ncells + (size_t)pb * NCB, NCB * 8u);
   }
 
+  // where the species pass finds line cell y of block m on line l
+  auto sp_line = [&](int m, int y, int l) {
+    int i, j, k;
+    G::cell(y, l, qtr, i, j, k);
+    return sp_line_base<NDIM, NX, NY, NZ, DIR>(K == 1 ? slot : pick(blk, m)) + DG::idx(i, j, k);
+  };
   if (K > 1 || P.fmode != 3) {
   // ---- stage
   if constexpr (K == 1) {
@@ -503,7 +509,8 @@ k_dir(const DevParams P, const double *__restrict__ SIG, double *__restrict__ AC
         else if (dp1 == 0.) flat = t0;
         else flat = rmax(t0, sDb[6 * G::SB + q - G::step]);
       }
-      if (K == 1 && P.sp_flat) P.sp_flat[sp_line_base<NDIM, NX, NY, NZ, DIR>(slot) + DG::idx(i, j, k)] = flat;
+      if (P.sp_flat)
+        seam_blocks<K, G::N0, false>(x, [&](int m, int y) { P.sp_flat[sp_line(m, y, l)] = flat; });
       eigen64<DIR>(Vc, e0, ar, st);
       ppm_states<DIR>(P, ar, Vm, Vc, Vp, [&](int n, int o) { return sDb[n * G::SB + q + o * G::step]; },
                       [&](int o) { return sQ[G::sidx(x + o, l)]; }, Vc[HGE], flat, dtn, delta, e0, Wp, Wm,
@@ -570,7 +577,7 @@ k_dir(const DevParams P, const double *__restrict__ SIG, double *__restrict__ AC
         sWm[qq * G::SC + t] = wm;
       }
       if (fb) cell_state();
-      if (K == 1 && P.sp_fb) P.sp_fb[sp_line_base<NDIM, NX, NY, NZ, DIR>(slot) + DG::idx(i, j, k)] = fb;
+      if (P.sp_fb) seam_blocks<K, G::N0, false>(x, [&](int m, int y) { P.sp_fb[sp_line(m, y, l)] = fb; });
     }
   };
   ar.bad = false;
@@ -606,11 +613,8 @@ k_dir(const DevParams P, const double *__restrict__ SIG, double *__restrict__ AC
     if (!P.use_aux_eint) fv = fe = 0.;
     sF[FEINT * G::SC + t] = fe;
     sF[FVOLU * G::SC + t] = fv;
-    if (K == 1 && P.sp_mf) {
-      int i, j, k;
-      G::cell(x, l, qtr, i, j, k);
-      P.sp_mf[sp_line_base<NDIM, NX, NY, NZ, DIR>(slot) + DG::idx(i, j, k)] = F[FDENS];
-    }
+    if (P.sp_mf)
+      seam_blocks<K, G::N0, true>(x, [&](int m, int y) { P.sp_mf[sp_line(m, y, l)] = F[FDENS]; });
   };
   ar.bad = false;
   for (int t = threadIdx.x; t < G::SC; t += blockDim.x) faces(ar, t);

@@ -361,6 +361,18 @@ template <int K> __device__ __forceinline__ int pick(const int (&blk)[K], int m)
   return b;
 }
 
+// Line cell x of a run's line (face x) as the blocks of the run know it:
+// f(m, xl) with xl relative to block m -- the block that holds it and, at the
+// seams, the neighbour whose line cells (faces) reach it (FACES: xl in
+// [0, N0], else [-1, N0]).
+template <int K, int N0, bool FACES, class F>
+__device__ __forceinline__ void seam_blocks(int x, F f) {
+  const int m = K == 1 || x < 0 ? 0 : (x >= K * N0 ? K - 1 : x / N0), xl = x - m * N0;
+  f(m, xl);
+  if (K > 1 && xl == 0 && m > 0) f(m - 1, N0);
+  if (K > 1 && !FACES && xl == N0 - 1 && m < K - 1) f(m + 1, -1);
+}
+
 // deterministic (max key, first index) reduction for the CFL step
 struct CflCand { double key, val; int idx; };
 __device__ __forceinline__ void cfl_merge(CflCand &a, const CflCand &b) {

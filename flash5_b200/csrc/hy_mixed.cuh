@@ -285,6 +285,13 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
   }
 
   auto fidx = [](int along, int t1, int t2) { return G::at(along, t1 + (DIR == 1 ? NY : NX) * t2, G::LC, 1); };
+  // where the species pass finds line cell y of block bm on line l
+  auto sp_line = [&](int bm, int y, int l) {
+    int i, j, k;
+    G::cell(y, l, qtr, i, j, k);
+    return sp_line_base<NDIM, NX, NY, NZ, DIR>(K == 1 ? (P.slot ? P.slot[b] : (int)blockIdx.x) : pick(blk, bm)) +
+           DirGeom<NDIM, NX, NY, NZ, double, DIR>::idx(i, j, k);
+  };
   if (P.fmode != 3) {
   // ---- A: stage the primitive stencil of every line (guard cells get the EOS)
   // Uniform 3D grids: the block's interior and the neighbours' slabs along
@@ -451,9 +458,8 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
       else if (dp1 == 0.) flat = t0;
       else flat = fmaxf(t0, sFlat[q - qs]);
     }
-    if (K == 1 && P.sp_flat)
-      P.sp_flat[sp_line_base<NDIM, NX, NY, NZ, DIR>(P.slot ? P.slot[b] : (int)blockIdx.x) + DirGeom<NDIM, NX, NY, NZ, double, DIR>::idx(i, j, k)] =
-          double(flat);
+    if (P.sp_flat)
+      seam_blocks<K, G::ND0, false>(x, [&](int bm, int y) { P.sp_flat[sp_line(bm, y, l)] = double(flat); });
     const int sl[6] = {0, 1, 2, 3, 4, 7};
     float lft[8], rgt[8], delW[8], W6[8];
 #pragma unroll
@@ -591,8 +597,7 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
 #pragma unroll
         for (int n = 0; n < 8; ++n) { dWm[n] = 0.f; dWp[n] = 0.f; }
       }
-      if (K == 1 && P.sp_fb)
-        P.sp_fb[sp_line_base<NDIM, NX, NY, NZ, DIR>(P.slot ? P.slot[b] : (int)blockIdx.x) + DirGeom<NDIM, NX, NY, NZ, double, DIR>::idx(i, j, k)] = fb;
+      if (P.sp_fb) seam_blocks<K, G::ND0, false>(x, [&](int bm, int y) { P.sp_fb[sp_line(bm, y, l)] = fb; });
     }
 #pragma unroll
     for (int qq = 0; qq < 6; ++qq) {
@@ -850,14 +855,13 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
     });
     __syncthreads();
   }
-  if (K == 1 && P.sp_mf) {        // face mass fluxes for the species pass
+  if (P.sp_mf) {                  // face mass fluxes for the species pass
     for (int t = threadIdx.x; t < G::SC; t += NT) {
-      int x, l, i, j, k;
+      int x, l;
       G::dec(t, G::LC, 1, x, l);
       if (x < 0) continue;
-      G::cell(x, l, i, j, k);
-      P.sp_mf[sp_line_base<NDIM, NX, NY, NZ, DIR>(P.slot ? P.slot[b] : (int)blockIdx.x) + DirGeom<NDIM, NX, NY, NZ, double, DIR>::idx(i, j, k)] =
-          sF[FDENS * G::SC + t];
+      const double mf = sF[FDENS * G::SC + t];
+      seam_blocks<K, G::ND0, true>(x, [&](int bm, int y) { P.sp_mf[sp_line(bm, y, l)] = mf; });
     }
   }
 

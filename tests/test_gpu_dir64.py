@@ -93,3 +93,24 @@ def test_exact_solver_runs_equal_one_block():
 def test_2d_equals_oracle(nb, opt):
     grid = UniformGrid(2, (nb, nb), (5, 3), bc=["reflecting", "outflow", "outflow", "reflecting"])
     _check_oracle(grid, abi.default_params(**opt), setups.four_quadrant(grid), 3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("prec,rs", [(abi.PREC_FP64, abi.RS_HLLC), (abi.PREC_MIXED, abi.RS_HLLC),
+                                     (abi.PREC_MIXED, abi.RS_EXACT)])
+def test_species_on_runs_equal_one_block(prec, rs):
+    """The per-line data the run kernels leave for the species pass (mass
+    fluxes, flattening, first-order flags, shared at the seams of a run)
+    against one block per CTA: bit for bit (FP64), to rounding (mixed)."""
+    grid = UniformGrid(3, (8, 8, 8), (8, 4, 4), bc=["outflow", "reflecting"] + ["periodic"] * 4, nspecies=2,
+                       nmass_scalars=1)
+    unk = setups.add_species(grid, setups.sod_axis(grid, axis=0))
+    h = Hydro(abi.default_params(precision=prec, riemann_solver=rs), grid)
+    runs, _ = _advance(h, None, grid, unk, 3)
+    one, _ = _advance(h, None, grid, unk, 3, blocks=range(grid.nblocks))
+    h.close()
+    if prec == abi.PREC_FP64:
+        assert np.array_equal(runs, one)
+    else:
+        # FP32 face values of separately compiled kernels: 1e-7 of values of order one
+        assert np.abs(grid.interior(runs)[..., grid.species] - grid.interior(one)[..., grid.species]).max() <= 1e-7
