@@ -75,6 +75,7 @@ struct flash_hy_ctx {
   int *d_level, *d_leaf, *d_parent, *d_slot, *d_at;
   int at_off[17], at_ext[17][3];
   int *d_leaves, nleaves;
+  int *d_guard, n_guard, n_guard_step;   // halo positions of a leaf's guard cells, those a step reads first
   int *d_lev_leaves[17], lev_leaves[17];
   int *d_lev_parents[17], lev_parents[17];
   int nparents;
@@ -410,6 +411,23 @@ static int amr_tables(const flash_hy_grid_desc *g, std::vector<int> &at, int off
   return 0;
 }
 
+// halo positions of a leaf's guard cells, those a step reads first (their
+// number in *step)
+template <int NDIM, int NX, int NY, int NZ>
+static std::vector<int> guard_cells(int *step) {
+  using H = Halo<NDIM, NX, NY, NZ>;
+  std::vector<int> v;
+  for (int pass = 0; pass < 2; ++pass) {
+    for (int h = 0; h < H::n; ++h) {
+      const int i = h % H::hx - 4, j = (h / H::hx) % H::hy - 4, k = NDIM > 2 ? h / (H::hx * H::hy) - 4 : 0;
+      const bool in = i >= 0 && i < NX && j >= 0 && j < NY && (NDIM < 3 || (k >= 0 && k < NZ));
+      if (!in && step_guard<NDIM, NX, NY, NZ>(i, j, k) == (pass == 0)) v.push_back(h);
+    }
+    if (pass == 0) *step = (int)v.size();
+  }
+  return v;
+}
+
 extern "C" int flash_hy_create(const flash_hy_params *params, const flash_hy_grid_desc *g, int device,
                                flash_hy_ctx **out) {
   if (!params || !g || !out) return FLASH_HY_ERR_BAD_ARG;
@@ -540,7 +558,13 @@ extern "C" int flash_hy_create(const flash_hy_params *params, const flash_hy_gri
     ALLOC(c->d_slot, g->nblocks * sizeof(int));
     ALLOC(c->d_at, amr_at.size() * sizeof(int));
     ALLOC(c->d_leaves, leaves.size() * sizeof(int));
-    bool ok = cudaMemcpy(c->d_level, g->block_level, g->nblocks * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
+    const std::vector<int> guard = g->ndim == 3 ? guard_cells<3, 8, 8, 8>(&c->n_guard_step)
+                                   : g->nxb == 8 ? guard_cells<2, 8, 8, 1>(&c->n_guard_step)
+                                                 : guard_cells<2, 16, 16, 1>(&c->n_guard_step);
+    c->n_guard = (int)guard.size();
+    ALLOC(c->d_guard, guard.size() * sizeof(int));
+    bool ok = cudaMemcpy(c->d_guard, guard.data(), guard.size() * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
+              cudaMemcpy(c->d_level, g->block_level, g->nblocks * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
               cudaMemcpy(c->d_leaf, amr_leaf.data(), g->nblocks * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
               cudaMemcpy(c->d_parent, amr_parent.data(), g->nblocks * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
               cudaMemcpy(c->d_slot, slot.data(), g->nblocks * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
@@ -684,7 +708,7 @@ extern "C" int flash_hy_destroy(flash_hy_ctx *c) {
   drop_graphs(c);
   ctx_free(c->d_stepdt);
   ctx_free(c->d_level); ctx_free(c->d_leaf); ctx_free(c->d_parent); ctx_free(c->d_slot); ctx_free(c->d_at);
-  ctx_free(c->d_leaves); ctx_free(c->d_lh); ctx_free(c->d_gp); ctx_free(c->d_pe); ctx_free(c->d_freg);
+  ctx_free(c->d_leaves); ctx_free(c->d_guard); ctx_free(c->d_lh); ctx_free(c->d_gp); ctx_free(c->d_pe); ctx_free(c->d_freg);
   for (int l = 0; l < 17; ++l) { ctx_free(c->d_lev_leaves[l]); ctx_free(c->d_lev_parents[l]); }
   ctx_free(c->d_owned); ctx_free(c->d_owned_mask); ctx_free(c->d_send); ctx_free(c->d_recv);
   ctx_free(c->d_inner); ctx_free(c->d_edge);
@@ -1095,7 +1119,7 @@ extern "C" int flash_hy_download(flash_hy_ctx *c, double *unk, int layout, int n
 // AMR: restriction (finest parents first), parent halos (coarsest first),
 // leaf guard cells; returns the number of launches, or -1 on a launch error
 template <int NDIM, int NX, int NY, int NZ>
-static int amr_guard_fill(flash_hy_ctx *c, const DevParams &P) {
+static int amr_guard_fill(flash_hy_ctx *c, const DevParams &P, bool step) {
   double *const *st = c->state[c->cur];
   int n = 0;
   for (int l = c->nlev - 1; l >= 1; --l) {
@@ -1112,15 +1136,17 @@ static int amr_guard_fill(flash_hy_ctx *c, const DevParams &P) {
                                                                              c->d_lev_parents[l]);
     ++n;
   }
-  k_leaf_halo<NDIM, NX, NY, NZ><<<c->nleaves, 256, 0, c->stream>>>(P, st[0], st[1], st[2], st[3], st[4], c->d_leaves);
+  k_leaf_halo<NDIM, NX, NY, NZ><<<c->nleaves, 256, 0, c->stream>>>(P, st[0], st[1], st[2], st[3], st[4], c->d_leaves,
+                                                                          c->d_guard, step ? c->n_guard_step : c->n_guard);
   ++n;
   return cudaGetLastError() == cudaSuccess ? n : -1;
 }
 
-static int amr_prepare(flash_hy_ctx *c, const DevParams &P) {
-  if (c->ndim == 2 && c->nx == 8) return amr_guard_fill<2, 8, 8, 1>(c, P);
-  if (c->ndim == 2 && c->nx == 16) return amr_guard_fill<2, 16, 16, 1>(c, P);
-  if (c->ndim == 3) return amr_guard_fill<3, 8, 8, 8>(c, P);
+// step: the leaves' guard cells that a step reads, else all of them
+static int amr_prepare(flash_hy_ctx *c, const DevParams &P, bool step) {
+  if (c->ndim == 2 && c->nx == 8) return amr_guard_fill<2, 8, 8, 1>(c, P, step);
+  if (c->ndim == 2 && c->nx == 16) return amr_guard_fill<2, 16, 16, 1>(c, P, step);
+  if (c->ndim == 3) return amr_guard_fill<3, 8, 8, 8>(c, P, step);
   return -1;
 }
 
@@ -1176,7 +1202,7 @@ static int enqueue_step(flash_hy_ctx *c, double dt, const int *d_list, int nlaun
   a.nlev = 0;
   int pre = 0;
   if (c->amr) {
-    pre = amr_prepare(c, a.P);
+    pre = amr_prepare(c, a.P, true);
     if (pre < 0) return fail(c, FLASH_HY_ERR_CUDA, "AMR guard-cell launch failed: %s", cudaGetErrorString(cudaGetLastError()));
     a.nlev = c->nlev;
     a.leaves = c->d_leaves;
@@ -1770,11 +1796,12 @@ done:
 // refinement criterion (gr_estimateError)
 // ---------------------------------------------------------------------------
 // the estimator of one variable for every node into the device array d_out
-static int estimate_into(flash_hy_ctx *c, int var, double refine_filter, double *d_out) {
+// (fill: the hierarchy's guard cells first)
+static int estimate_into(flash_hy_ctx *c, int var, double refine_filter, double *d_out, bool fill) {
   CUDA_OK(c, cudaMemsetAsync(d_out, 0, (size_t)c->nblocks * sizeof(double), c->stream));
   ErrArgs a;
   fill_devparams(c, a.P);
-  if (c->amr && amr_prepare(c, a.P) < 0)
+  if (fill && c->amr && amr_prepare(c, a.P, false) < 0)
     return fail(c, FLASH_HY_ERR_CUDA, "AMR guard-cell launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   a.var = var;
   a.filter = refine_filter;
@@ -1799,12 +1826,12 @@ extern "C" int flash_hy_mark_refine_tree(flash_hy_ctx *c, int nvar, const int *v
   CUDA_OK(c, cudaSetDevice(c->device));
   double *d_err = nullptr, *d_cut = nullptr;
   int rc = 0, trc = 0;
-  if (cudaMalloc((void **)&d_err, (size_t)nvar * c->nblocks * sizeof(double)) != cudaSuccess ||
-      cudaMalloc((void **)&d_cut, 2 * (size_t)nvar * sizeof(double)) != cudaSuccess) {
-    cudaFree(d_err);
+  if (ctx_alloc((void **)&d_err, (size_t)nvar * c->nblocks * sizeof(double)) != cudaSuccess ||
+      ctx_alloc((void **)&d_cut, 2 * (size_t)nvar * sizeof(double)) != cudaSuccess) {
+    ctx_free(d_err);
     return fail(c, FLASH_HY_ERR_CUDA, "mark_refine_tree allocation%s", "");
   }
-  for (int v = 0; v < nvar && !rc; ++v) rc = estimate_into(c, vars[v], refine_filter, d_err + (size_t)v * c->nblocks);
+  for (int v = 0; v < nvar && !rc; ++v) rc = estimate_into(c, vars[v], refine_filter, d_err + (size_t)v * c->nblocks, v == 0);
   if (!rc) {
     std::vector<double> cut(2 * (size_t)nvar);
     for (int v = 0; v < nvar; ++v) { cut[v] = refine_cutoff[v]; cut[nvar + v] = derefine_cutoff[v]; }
@@ -1823,6 +1850,7 @@ extern "C" int flash_hy_mark_refine_tree(flash_hy_ctx *c, int nvar, const int *v
       }
       for (int d = 0; d < 3; ++d) a.periodic[d] = d < c->ndim && c->bc[2 * d] == FLASH_HY_BC_PERIODIC;
       a.stream = c->stream; a.cap = cap;
+      a.alloc = ctx_alloc; a.release = ctx_free;
       a.new_n = new_n; a.new_levels = new_levels; a.new_coords = new_coords; a.new_parent = new_parent;
       a.src = src; a.how = how;
       if (cap > 0 && (!new_levels || !new_coords || !new_parent || !src || !how)) trc = -4;
@@ -1833,8 +1861,8 @@ extern "C" int flash_hy_mark_refine_tree(flash_hy_ctx *c, int nvar, const int *v
     }
   }
   cudaStreamSynchronize(c->stream);
-  cudaFree(d_err);
-  cudaFree(d_cut);
+  ctx_free(d_err);
+  ctx_free(d_cut);
   return rc;
 }
 
@@ -1848,7 +1876,7 @@ extern "C" int flash_hy_estimate_error(flash_hy_ctx *c, int var, double refine_f
   CUDA_OK(c, cudaMemsetAsync(c->d_err, 0, (size_t)c->nblocks * sizeof(double), c->stream));
   ErrArgs a;
   fill_devparams(c, a.P);
-  if (c->amr && amr_prepare(c, a.P) < 0)
+  if (c->amr && amr_prepare(c, a.P, false) < 0)
     return fail(c, FLASH_HY_ERR_CUDA, "AMR guard-cell launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   a.var = var;
   a.filter = refine_filter;
@@ -1887,7 +1915,7 @@ extern "C" int flash_hy_regrid(flash_hy_ctx *old, flash_hy_ctx *nw, int n, const
   CUDA_OK(nw, cudaStreamSynchronize(nw->stream));
   RegridArgs a;
   fill_devparams(old, a.Po);
-  if (amr_prepare(old, a.Po) < 0)
+  if (amr_prepare(old, a.Po, false) < 0)
     return fail(old, FLASH_HY_ERR_CUDA, "AMR guard-cell launch failed: %s", cudaGetErrorString(cudaGetLastError()));
   fill_devparams(nw, a.Pn);
   for (int v = 0; v < 5; ++v) a.Pn.s_out[v] = nw->state[nw->cur][v];

@@ -121,6 +121,9 @@ struct TreeArgs {
   int at_ext[17][3];
   int periodic[3];
   cudaStream_t stream;
+  // the contexts' cached device memory (a call's dozen work buffers)
+  cudaError_t (*alloc)(void **p, size_t bytes);
+  void (*release)(void *p);
   int cap;
   int *new_n, *new_levels, *new_coords, *new_parent, *src, *how;
 };

@@ -38,24 +38,34 @@ __global__ void __launch_bounds__(256) k_estimate_error(const DevParams P, int v
   const bool parent = amr && !P.leaf[b];
   const int l = amr ? P.blk_level[b] : 1;
   const int3 bc = blk_coords(P, b);
+  // the stored arrays the variable needs: one, or rho and e for the pressure
+  const bool pres = var == FLASH_HY_REFVAR_PRES, eint = var == FLASH_HY_REFVAR_EINT;
+  const int comp = var == FLASH_HY_REFVAR_DENS ? 0
+                   : (var == FLASH_HY_REFVAR_VELX ? 1 : (var == FLASH_HY_REFVAR_VELY ? 2 : (var == FLASH_HY_REFVAR_VELZ ? 3 : 4)));
+  constexpr int NCB = NX * NY * NZ;
   for (int h = threadIdx.x; h < H::n; h += blockDim.x) {
     const int li = h % H::hx - 4, lj = NDIM > 1 ? (h / H::hx) % H::hy - 4 : 0;
     const int lk = NDIM > 2 ? h / (H::hx * H::hy) - 4 : 0;
+    const bool inside = is_inside<NDIM, NX, NY, NZ>(li, lj, lk);
     double v;
     if (parent) {
       const double *g = P.gp + (size_t)P.slot[b] * 6 * H::n;
-      const double rho = g[h], vx = g[H::n + h], vy = g[2 * H::n + h], vz = g[3 * H::n + h];
-      double e = g[4 * H::n + h];
-      if (!is_inside<NDIM, NX, NY, NZ>(li, lj, lk) && (var == FLASH_HY_REFVAR_PRES || var == FLASH_HY_REFVAR_EINT)) {
-        const double E = g[5 * H::n + h];
+      v = g[comp * H::n + h];
+      if (!inside && (pres || eint)) {
+        const double vx = g[H::n + h], vy = g[2 * H::n + h], vz = g[3 * H::n + h], E = g[5 * H::n + h];
         const double ekin = 0.5 * (vx * vx + vy * vy + vz * vz);
-        if (E - ekin > rmax(P.smalle, P.eswitch * ekin)) e = E - ekin;
+        if (E - ekin > rmax(P.smalle, P.eswitch * ekin)) v = E - ekin;
       }
-      v = refvar(var, rho, vx, vy, vz, e, P.gam1inv);
+      if (pres) v = g[h] * v * P.gam1inv;
+    } else if (amr) {
+      const double *g = P.lh + (size_t)P.slot[b] * 5 * H::n + h;
+      const size_t o = (size_t)b * NCB + (size_t)((lk * NY + lj) * NX + li);
+      v = inside ? __ldg(P.s_in[comp] + o) : g[comp * H::n];
+      if (pres) v = (inside ? __ldg(P.s_in[0] + o) : g[0]) * v * P.gam1inv;
     } else {
       double V[8];
       load_prim<NDIM, NX, NY, NZ, false>(P, b, bc, li, lj, lk, V);
-      v = var == FLASH_HY_REFVAR_PRES ? V[HP] : refvar(var, V[HD], V[HVX], V[HVY], V[HVZ], V[HEI], P.gam1inv);
+      v = pres ? V[HP] : refvar(var, V[HD], V[HVX], V[HVY], V[HVZ], V[HEI], P.gam1inv);
     }
     sV[h] = v;
   }

@@ -302,15 +302,15 @@ int tree_update_dev(const TreeArgs &a) {
   do {                                            \
     if ((x) != cudaSuccess) { rc = -2; goto out; } \
   } while (0)
-  TCHK(cudaMalloc((void **)&T, ntab));
-  TCHK(cudaMalloc((void **)&flag, ntab));
-  TCHK(cudaMalloc((void **)&cand, ntab));
-  TCHK(cudaMalloc((void **)&refine, a.nblocks));
-  TCHK(cudaMalloc((void **)&deref, a.nblocks));
-  TCHK(cudaMalloc((void **)&d_changed, 2 * sizeof(int)));
+  TCHK(a.alloc((void **)&T, ntab));
+  TCHK(a.alloc((void **)&flag, ntab));
+  TCHK(a.alloc((void **)&cand, ntab));
+  TCHK(a.alloc((void **)&refine, a.nblocks));
+  TCHK(a.alloc((void **)&deref, a.nblocks));
+  TCHK(a.alloc((void **)&d_changed, 2 * sizeof(int)));
   d_bad = d_changed + 1;
-  TCHK(cudaMalloc((void **)&sflag, (nslots + 1) * sizeof(int)));
-  TCHK(cudaMalloc((void **)&sidx, (nslots + 1) * sizeof(int)));
+  TCHK(a.alloc((void **)&sflag, (nslots + 1) * sizeof(int)));
+  TCHK(a.alloc((void **)&sidx, (nslots + 1) * sizeof(int)));
   TCHK(cudaMemsetAsync(T, 0, ntab, st));
   TCHK(cudaMemsetAsync(flag, 0, ntab, st));
   TCHK(cudaMemsetAsync(cand, 0, ntab, st));
@@ -347,14 +347,14 @@ int tree_update_dev(const TreeArgs &a) {
   k_slot_flags<<<grid(nslots), B, 0, st>>>(V, nslots, T, sflag);
   TCHK(cudaGetLastError());
   TCHK(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, sflag, sidx, (int)(nslots + 1), st));
-  TCHK(cudaMalloc(&tmp, tmp_bytes));
+  TCHK(a.alloc(&tmp, tmp_bytes));
   TCHK(cudaMemsetAsync(sflag + nslots, 0, sizeof(int), st));
   TCHK(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, sflag, sidx, (int)(nslots + 1), st));
   TCHK(cudaMemcpyAsync(&n, sidx + nslots, sizeof(int), cudaMemcpyDeviceToHost, st));
   TCHK(cudaStreamSynchronize(st));
   *a.new_n = n;
   if (n > a.cap) { rc = -4; goto out; }
-  TCHK(cudaMalloc((void **)&o_lev, (size_t)n * 7 * sizeof(int)));
+  TCHK(a.alloc((void **)&o_lev, (size_t)n * 7 * sizeof(int)));
   o_coord = o_lev + n; o_par = o_coord + 3 * (size_t)n; o_src = o_par + n; o_how = o_src + n;
   k_emit<<<grid(nslots), B, 0, st>>>(V, nslots, sflag, sidx, T, a.old_at, a.leaf, o_lev, o_coord, o_par, o_src,
                                      o_how, d_bad);
@@ -369,8 +369,9 @@ int tree_update_dev(const TreeArgs &a) {
   if (h_bad) rc = -5;
 out:
 #undef TCHK
-  cudaFree(T); cudaFree(flag); cudaFree(cand); cudaFree(refine); cudaFree(deref); cudaFree(d_changed);
-  cudaFree(sflag); cudaFree(sidx); cudaFree(o_lev); cudaFree(tmp);
+  cudaStreamSynchronize(st);               // an early exit may leave kernels in flight
+  a.release(T); a.release(flag); a.release(cand); a.release(refine); a.release(deref); a.release(d_changed);
+  a.release(sflag); a.release(sidx); a.release(o_lev); a.release(tmp);
   return rc;
 }
 
