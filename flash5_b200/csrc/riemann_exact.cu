@@ -485,142 +485,220 @@ __global__ void k_make_samples(const double *S, const double *out, long n, float
 }
 
 // ---------------------------------------------------------------------------
-// FP32 forward/backward of one minibatch (MSE, mean over the batch); each
-// CTA handles TS samples and adds its gradient into G (atomics)
+// FP32 forward/backward of one minibatch (MSE, mean over the batch).  A CTA
+// takes TS samples and writes its share of the gradient and of the sum of
+// squared residuals to its row of `part` ([CTAs][PSTRIDE]; no atomics, so a
+// run repeats bit for bit); k_reduce or k_adam adds the rows.  The 64 x 64
+// products run as register tiles from shared memory: 2 samples x 4 units per
+// thread forward and for dH1, 4 x 4 for dW2.  One wave at 4096 samples (128
+// CTAs); bound by the latency of its five phases.
+// 24 batches of 4096, two epochs: 1.46-2.11 ms (scalar loads, 5,000 atomics per
+// CTA, three launches and a cudaMalloc per call) -> 1.19 ms.
 // ---------------------------------------------------------------------------
-constexpr int TS = 32, TRAIN_THREADS = 256;
+constexpr int TS = 32, TRAIN_THREADS = 256, PSTRIDE = (NPARAM + 1 + 31) / 32 * 32;
+constexpr int WS = NH + 4;                 // row strides that keep float4 rows aligned, banks spread
+struct __align__(16) TrainSmem {
+  float W2[NH][WS], W2T[NH][WS];           // [u][j], [j][u]
+  float H1[TS][WS], H2[TS][WS];            // activations, then H2 = dL/dh2
+  float W1[NH * NIN], X[TS][NIN];
+  float B1[NH], B2[NH], W3[NH], D[TS], R[TS];
+};
 
 __global__ void __launch_bounds__(TRAIN_THREADS) k_grad(const float *__restrict__ w, const float *__restrict__ X,
                                                         const float *__restrict__ T, const int *__restrict__ idx, int nb,
-                                                        float inv_batch, float *__restrict__ G, float *__restrict__ loss) {
-  __shared__ float sW1[NH * NIN], sB1[NH], sW2[NH * NH], sB2[NH], sW3[NH];
-  __shared__ float sX[TS][NIN], sH1[TS][NH + 1], sH2[TS][NH + 1], sD[TS];
-  __shared__ float gW1[NH * NIN], gB1[NH], gW3[NH], gB2[NH];
+                                                        float inv_batch, float *__restrict__ part) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  TrainSmem &s = *reinterpret_cast<TrainSmem *>(smem_raw);
   const int tid = threadIdx.x;
-  for (int t = tid; t < NH * NIN; t += TRAIN_THREADS) { sW1[t] = w[OFF_W1 + t]; gW1[t] = 0.f; }
-  for (int t = tid; t < NH * NH; t += TRAIN_THREADS) sW2[t] = w[OFF_W2 + t];
-  for (int t = tid; t < NH; t += TRAIN_THREADS) {
-    sB1[t] = w[OFF_B1 + t]; sB2[t] = w[OFF_B2 + t]; sW3[t] = w[OFF_W3 + t];
-    gB1[t] = 0.f; gW3[t] = 0.f; gB2[t] = 0.f;
+  float *G = part + (size_t)blockIdx.x * PSTRIDE;
+  // the CTA's first tile writes its row, later ones (batches beyond
+  // GRAD_CTAS tiles) add to it
+  bool first = true;
+  auto put = [&](int t, float x) { G[t] = first ? x : G[t] + x; };
+  for (int t = tid; t < NH * NIN; t += TRAIN_THREADS) s.W1[t] = w[OFF_W1 + t];
+  for (int t = tid; t < NH * NH; t += TRAIN_THREADS) {
+    const float v = w[OFF_W2 + t];
+    s.W2[t / NH][t % NH] = v;
+    s.W2T[t % NH][t / NH] = v;
   }
+  if (tid < NH) { s.B1[tid] = w[OFF_B1 + tid]; s.B2[tid] = w[OFF_B2 + tid]; s.W3[tid] = w[OFF_W3 + tid]; }
   const float b3 = w[OFF_B3];
-  const int s0 = blockIdx.x * TS;
+  for (int s0 = blockIdx.x * TS; s0 < nb; s0 += gridDim.x * TS, first = false) {
   const int ns = min(TS, nb - s0);
-  for (int t = tid; t < TS * NIN; t += TRAIN_THREADS) {
-    int s = t / NIN, k = t % NIN;
-    sX[s][k] = s < ns ? X[(long)idx[s0 + s] * NIN + k] : 0.f;
+  __syncthreads();                         // the previous tile's last reads
+  {
+    const int q = tid / NIN, k = tid % NIN;                       // TS * NIN = TRAIN_THREADS
+    s.X[q][k] = q < ns ? X[(long)idx[s0 + q] * NIN + k] : 0.f;
   }
   __syncthreads();
-  // forward
-  for (int t = tid; t < TS * NH; t += TRAIN_THREADS) {
-    int s = t / NH, u = t % NH;
-    float a = sB1[u];
+  // thread tile of the forward products: samples 2 sp, 2 sp + 1, units 4 ug .. 4 ug + 3
+  const int sp = tid >> 4, ug = tid & 15;
+  {
+    float x[2][NIN];
 #pragma unroll
-    for (int k = 0; k < NIN; ++k) a += sW1[u * NIN + k] * sX[s][k];
-    sH1[s][u] = fmaxf(a, 0.f);
-  }
-  __syncthreads();
-  for (int t = tid; t < TS * NH; t += TRAIN_THREADS) {
-    int s = t / NH, u = t % NH;
-    float a = sB2[u];
-    for (int j = 0; j < NH; ++j) a += sW2[u * NH + j] * sH1[s][j];
-    sH2[s][u] = fmaxf(a, 0.f);
-  }
-  __syncthreads();
-  // output and dL/dy per sample (one warp per group of samples)
-  float lsum = 0.f;
-  for (int s = tid >> 5; s < TS; s += TRAIN_THREADS / 32) {
-    float a = 0.f;
-    for (int u = tid & 31; u < NH; u += 32) a += sW3[u] * sH2[s][u];
+    for (int e = 0; e < 2; ++e)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if ((tid & 31) == 0) {
-      float y = a + b3;
-      float r = s < ns ? y - T[idx[s0 + s]] : 0.f;
-      sD[s] = 2.f * r * inv_batch;
-      lsum += r * r;
+      for (int k = 0; k < NIN; ++k) x[e][k] = s.X[2 * sp + e][k];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const int u = 4 * ug + v;
+      float a0 = s.B1[u], a1 = a0;
+#pragma unroll
+      for (int k = 0; k < NIN; ++k) { a0 += s.W1[u * NIN + k] * x[0][k]; a1 += s.W1[u * NIN + k] * x[1][k]; }
+      s.H1[2 * sp][u] = fmaxf(a0, 0.f);
+      s.H1[2 * sp + 1][u] = fmaxf(a1, 0.f);
     }
   }
   __syncthreads();
-  // dH2 (in place over sH2 after using it for dW3)
-  for (int u = tid; u < NH; u += TRAIN_THREADS) {
-    float gw = 0.f;
-    for (int s = 0; s < TS; ++s) gw += sD[s] * sH2[s][u];
-    gW3[u] = gw;
-  }
-  __syncthreads();
-  for (int t = tid; t < TS * NH; t += TRAIN_THREADS) {
-    int s = t / NH, u = t % NH;
-    sH2[s][u] = sH2[s][u] > 0.f ? sD[s] * sW3[u] : 0.f;
-  }
-  __syncthreads();
-  // dW2[u][j] = sum_s dH2[s][u] H1[s][j], db2
-  for (int t = tid; t < NH * NH; t += TRAIN_THREADS) {
-    int u = t / NH, j = t % NH;
-    float a = 0.f;
-    for (int s = 0; s < TS; ++s) a += sH2[s][u] * sH1[s][j];
-    atomicAdd(&G[OFF_W2 + t], a);
-  }
-  for (int u = tid; u < NH; u += TRAIN_THREADS) {
-    float a = 0.f;
-    for (int s = 0; s < TS; ++s) a += sH2[s][u];
-    gB2[u] = a;
-  }
-  // dH1 = (dH2 W2) relu'(H1), written into a register pass then sH1
-  __syncthreads();
-  float dh1[TS * NH / TRAIN_THREADS];
+  {
+    float a[2][4];
 #pragma unroll
-  for (int q = 0; q < TS * NH / TRAIN_THREADS; ++q) {
-    int t = tid + q * TRAIN_THREADS;
-    int s = t / NH, j = t % NH;
-    float a = 0.f;
-    for (int u = 0; u < NH; ++u) a += sH2[s][u] * sW2[u * NH + j];
-    dh1[q] = sH1[s][j] > 0.f ? a : 0.f;
+    for (int v = 0; v < 4; ++v) a[0][v] = a[1][v] = s.B2[4 * ug + v];
+#pragma unroll 8
+    for (int j = 0; j < NH; ++j) {
+      const float4 q = *reinterpret_cast<const float4 *>(&s.W2T[j][4 * ug]);
+      const float h0 = s.H1[2 * sp][j], h1 = s.H1[2 * sp + 1][j];
+      a[0][0] += q.x * h0; a[0][1] += q.y * h0; a[0][2] += q.z * h0; a[0][3] += q.w * h0;
+      a[1][0] += q.x * h1; a[1][1] += q.y * h1; a[1][2] += q.z * h1; a[1][3] += q.w * h1;
+    }
+    float y[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      y[e] = 0.f;
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        a[e][v] = fmaxf(a[e][v], 0.f);
+        s.H2[2 * sp + e][4 * ug + v] = a[e][v];
+        y[e] += s.W3[4 * ug + v] * a[e][v];
+      }
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) y[e] += __shfl_xor_sync(0xffffffffu, y[e], o);    // the 16 lanes of the sample
+      if (ug == 0) {
+        const int q = 2 * sp + e;
+        const float r = q < ns ? y[e] + b3 - T[idx[s0 + q]] : 0.f;
+        s.D[q] = 2.f * r * inv_batch;
+        s.R[q] = r * r;
+      }
+    }
+  }
+  __syncthreads();
+  // dW3 and the sums, before H2 becomes dL/dh2
+  if (tid < NH) {
+    float g = 0.f;
+#pragma unroll 8
+    for (int q = 0; q < TS; ++q) g += s.D[q] * s.H2[q][tid];
+    put(OFF_W3 + tid, g);
+  } else if (tid < NH + 32) {
+    float d = s.D[tid - NH], r = s.R[tid - NH];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      d += __shfl_xor_sync(0xffffffffu, d, o);
+      r += __shfl_xor_sync(0xffffffffu, r, o);
+    }
+    if (tid == NH) { put(OFF_B3, d); put(NPARAM, r); }
   }
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < TS * NH / TRAIN_THREADS; ++q) {
-    int t = tid + q * TRAIN_THREADS;
-    sH1[t / NH][t % NH] = dh1[q];
+  for (int e = 0; e < 2; ++e)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      float &h = s.H2[2 * sp + e][4 * ug + v];
+      h = h > 0.f ? s.D[2 * sp + e] * s.W3[4 * ug + v] : 0.f;
+    }
+  __syncthreads();
+  // dW2[u][j] = sum_s dh2[s][u] h1[s][j]: units 4 sp .. , inputs 4 ug ..; db2
+  {
+    float a[4][4] = {};
+#pragma unroll 4
+    for (int q = 0; q < TS; ++q) {
+      const float4 d = *reinterpret_cast<const float4 *>(&s.H2[q][4 * sp]);
+      const float4 h = *reinterpret_cast<const float4 *>(&s.H1[q][4 * ug]);
+      const float dv[4] = {d.x, d.y, d.z, d.w}, hv[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+      for (int m = 0; m < 4; ++m)
+#pragma unroll
+        for (int n = 0; n < 4; ++n) a[m][n] += dv[m] * hv[n];
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m)
+#pragma unroll
+      for (int n = 0; n < 4; ++n) put(OFF_W2 + (4 * sp + m) * NH + 4 * ug + n, a[m][n]);
+  }
+  if (tid < NH) {
+    float g = 0.f;
+#pragma unroll 8
+    for (int q = 0; q < TS; ++q) g += s.H2[q][tid];
+    put(OFF_B2 + tid, g);
+  }
+  // dH1 = (dH2 W2) relu'(H1)
+  {
+    float a[2][4] = {};
+#pragma unroll 8
+    for (int u = 0; u < NH; ++u) {
+      const float4 q = *reinterpret_cast<const float4 *>(&s.W2[u][4 * ug]);
+      const float d0 = s.H2[2 * sp][u], d1 = s.H2[2 * sp + 1][u];
+      a[0][0] += q.x * d0; a[0][1] += q.y * d0; a[0][2] += q.z * d0; a[0][3] += q.w * d0;
+      a[1][0] += q.x * d1; a[1][1] += q.y * d1; a[1][2] += q.z * d1; a[1][3] += q.w * d1;
+    }
+    __syncthreads();                       // every thread is done reading H1 (dW2)
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        float &h = s.H1[2 * sp + e][4 * ug + v];
+        h = h > 0.f ? a[e][v] : 0.f;
+      }
   }
   __syncthreads();
   for (int t = tid; t < NH * NIN; t += TRAIN_THREADS) {
-    int j = t / NIN, k = t % NIN;
+    const int j = t / NIN, k = t % NIN;
     float a = 0.f;
-    for (int s = 0; s < TS; ++s) a += sH1[s][j] * sX[s][k];
-    gW1[t] = a;
+#pragma unroll 8
+    for (int q = 0; q < TS; ++q) a += s.H1[q][j] * s.X[q][k];
+    put(OFF_W1 + t, a);
   }
-  for (int j = tid; j < NH; j += TRAIN_THREADS) {
+  if (tid < NH) {
     float a = 0.f;
-    for (int s = 0; s < TS; ++s) a += sH1[s][j];
-    gB1[j] = a;
+#pragma unroll 8
+    for (int q = 0; q < TS; ++q) a += s.H1[q][tid];
+    put(OFF_B1 + tid, a);
   }
-  __syncthreads();
-  for (int t = tid; t < NH * NIN; t += TRAIN_THREADS) atomicAdd(&G[OFF_W1 + t], gW1[t]);
-  for (int t = tid; t < NH; t += TRAIN_THREADS) {
-    atomicAdd(&G[OFF_B1 + t], gB1[t]);
-    atomicAdd(&G[OFF_B2 + t], gB2[t]);
-    atomicAdd(&G[OFF_W3 + t], gW3[t]);
   }
-  if (tid == 0) {
-    float a = 0.f;
-    for (int s = 0; s < TS; ++s) a += sD[s];
-    atomicAdd(&G[OFF_B3], a);
-  }
-  // loss (sum of squared residuals of this CTA)
-  if ((tid & 31) == 0) atomicAdd(loss, lsum);
 }
 
-__global__ void k_adam(float *w, float *m, float *v, const float *G, int step, float lr, float b1, float b2, float eps) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= NPARAM) return;
-  float g = G[t];
+// sum of column t of part's n rows over the 8 lanes that share it (every
+// lane returns it; a fixed order)
+__device__ __forceinline__ float column_sum(const float *__restrict__ part, int n, int t, int lane8) {
+  float a = 0.f;
+#pragma unroll 4
+  for (int r = lane8; r < n; r += 8) a += part[(size_t)r * PSTRIDE + t];
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  return a;
+}
+
+// gradient G[NPARAM] and summed squared residuals from k_grad's rows
+__global__ void __launch_bounds__(256) k_reduce(const float *__restrict__ part, int n, float *G, float *loss) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x, t = min(q >> 3, NPARAM);
+  const float a = column_sum(part, n, t, q & 7);
+  if ((q & 7) == 0 && q >> 3 <= NPARAM) { if (t < NPARAM) G[t] = a; else *loss = a; }
+}
+
+// Adam on the summed gradient; the last column adds the batch's squared
+// residuals to the epoch's
+__global__ void __launch_bounds__(256) k_adam(float *w, float *m, float *v, const float *__restrict__ part, int n,
+                                              float *loss, int step, float lr, float b1, float b2, float eps) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x, t = min(q >> 3, NPARAM);
+  const float g = column_sum(part, n, t, q & 7);
+  if ((q & 7) != 0 || q >> 3 > NPARAM) return;
+  if (t == NPARAM) { *loss += g; return; }
   m[t] = b1 * m[t] + (1.f - b1) * g;
   v[t] = b2 * v[t] + (1.f - b2) * g * g;
   float mh = m[t] / (1.f - powf(b1, (float)step));
   float vh = v[t] / (1.f - powf(b2, (float)step));
   w[t] -= lr * mh / (sqrtf(vh) + eps);
 }
+constexpr int RED_GRID = ((NPARAM + 1) * 8 + 255) / 256;
 
 __global__ void k_shuffle_idx(int *idx, int n, uint64_t seed) {
   // one random key per sample, then the host sorts nothing: a multiplicative
@@ -648,6 +726,9 @@ struct flash_hy_rsolver {
   MlpPacked *packed;            // BF16 inference copy of w
   int *queue, *qcount;          // fallback queue of the learned path
   long qcap;
+  float *part;                  // k_grad's rows [GRAD_CTAS][PSTRIDE]
+  int *idx;                     // train: the epoch's sample order
+  long idx_cap;
   unsigned *status;
   int step;
   int infer;                    // FLASH_HY_INFER_TCGEN05 or FLASH_HY_INFER_WARP_MMA
@@ -666,6 +747,9 @@ static int grid_for(long n, int threads) {
   if (g > 148L * 16) g = 148L * 16;
   return (int)(g > 0 ? g : 1);
 }
+
+constexpr long GRAD_CTAS = 296;         // two per SM
+static long grad_ctas(long nb) { const long t = (nb + TS - 1) / TS; return t < GRAD_CTAS ? t : GRAD_CTAS; }
 
 static int repack(flash_hy_rsolver *r) {
   k_pack_mlp<<<1, 256, 0, r->stream>>>(r->w, r->packed);
@@ -707,14 +791,21 @@ extern "C" int flash_hy_rsolver_create(int device, flash_hy_rsolver **out) {
   r->device = device;
   RS_CUDA(cudaSetDevice(device));
   RS_CUDA(cudaStreamCreateWithFlags(&r->stream, cudaStreamNonBlocking));
-  RS_CUDA(cudaMalloc(&r->w, NPARAM * sizeof(float)));
-  RS_CUDA(cudaMalloc(&r->m, NPARAM * sizeof(float)));
-  RS_CUDA(cudaMalloc(&r->v, NPARAM * sizeof(float)));
-  RS_CUDA(cudaMalloc(&r->G, NPARAM * sizeof(float)));
-  RS_CUDA(cudaMalloc(&r->loss, sizeof(float)));
-  RS_CUDA(cudaMalloc(&r->status, sizeof(unsigned)));
-  RS_CUDA(cudaMalloc(&r->qcount, sizeof(int)));
-  RS_CUDA(cudaMalloc(&r->packed, sizeof(MlpPacked)));
+  // one allocation, w at its start
+  const size_t row = PSTRIDE * sizeof(float);
+  char *mem = nullptr;
+  RS_CUDA(cudaMalloc((void **)&mem, (4 + GRAD_CTAS) * row + 256 + sizeof(MlpPacked)));
+  r->w = (float *)mem;
+  r->m = (float *)(mem + row);
+  r->v = (float *)(mem + 2 * row);
+  r->G = (float *)(mem + 3 * row);
+  r->part = (float *)(mem + 4 * row);
+  mem += (4 + GRAD_CTAS) * row;
+  r->packed = (MlpPacked *)mem;
+  mem += (sizeof(MlpPacked) + 15) / 16 * 16;
+  r->loss = (float *)mem;
+  r->status = (unsigned *)(mem + 16);
+  r->qcount = (int *)(mem + 32);
   RS_CUDA(cudaMemset(r->m, 0, NPARAM * sizeof(float)));
   RS_CUDA(cudaMemset(r->v, 0, NPARAM * sizeof(float)));
   RS_CUDA(cudaMemset(r->status, 0, sizeof(unsigned)));
@@ -737,6 +828,7 @@ extern "C" int flash_hy_rsolver_create(int device, flash_hy_rsolver **out) {
   r->tc_grid = sms * occ_s;
   r->tc_grid_p = sms * occ_p;
   r->infer = FLASH_HY_INFER_TCGEN05;
+  RS_CUDA(cudaFuncSetAttribute(k_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem)));
   return repack(r);
 }
 
@@ -755,8 +847,7 @@ extern "C" int flash_hy_rsolver_destroy(flash_hy_rsolver *r) {
   if (!r) return FLASH_HY_ERR_BAD_ARG;
   cudaSetDevice(r->device);
   if (r->stream) cudaStreamSynchronize(r->stream);
-  cudaFree(r->w); cudaFree(r->m); cudaFree(r->v); cudaFree(r->G); cudaFree(r->loss); cudaFree(r->status);
-  cudaFree(r->queue); cudaFree(r->qcount); cudaFree(r->packed);
+  cudaFree(r->w); cudaFree(r->queue); cudaFree(r->idx);
   if (r->stream) cudaStreamDestroy(r->stream);
   free(r);
   return 0;
@@ -836,9 +927,8 @@ extern "C" int flash_hy_rsolver_grad(flash_hy_rsolver *r, const float *d_x, cons
                                      float *h_grad, float *h_loss) {
   if (!r || !d_x || !d_t || !d_idx || nb <= 0) return FLASH_HY_ERR_BAD_ARG;
   RS_CUDA(cudaSetDevice(r->device));
-  RS_CUDA(cudaMemsetAsync(r->G, 0, NPARAM * sizeof(float), r->stream));
-  RS_CUDA(cudaMemsetAsync(r->loss, 0, sizeof(float), r->stream));
-  k_grad<<<(nb + TS - 1) / TS, TRAIN_THREADS, 0, r->stream>>>(r->w, d_x, d_t, d_idx, nb, 1.f / nb, r->G, r->loss);
+  k_grad<<<(int)grad_ctas(nb), TRAIN_THREADS, sizeof(TrainSmem), r->stream>>>(r->w, d_x, d_t, d_idx, nb, 1.f / nb, r->part);
+  k_reduce<<<RED_GRID, 256, 0, r->stream>>>(r->part, (int)grad_ctas(nb), r->G, r->loss);
   RS_CUDA(cudaGetLastError());
   if (h_grad) RS_CUDA(cudaMemcpyAsync(h_grad, r->G, NPARAM * sizeof(float), cudaMemcpyDeviceToHost, r->stream));
   if (h_loss) RS_CUDA(cudaMemcpyAsync(h_loss, r->loss, sizeof(float), cudaMemcpyDeviceToHost, r->stream));
@@ -853,27 +943,31 @@ extern "C" int flash_hy_rsolver_train(flash_hy_rsolver *r, const float *d_x, con
                                       int batch, float lr, float *loss_out) {
   if (!r || !d_x || !d_t || ns < batch || batch <= 0 || epochs <= 0) return FLASH_HY_ERR_BAD_ARG;
   RS_CUDA(cudaSetDevice(r->device));
-  int *idx;
-  RS_CUDA(cudaMalloc(&idx, ns * sizeof(int)));
+  if (r->idx_cap < ns) {
+    if (r->idx) { RS_CUDA(cudaStreamSynchronize(r->stream)); cudaFree(r->idx); r->idx = nullptr; r->idx_cap = 0; }
+    RS_CUDA(cudaMalloc((void **)&r->idx, ns * sizeof(int)));
+    r->idx_cap = ns;
+  }
+  int *idx = r->idx;
+  const int ctas = (int)grad_ctas(batch);
   float last = 0.f;
   long nbat = ns / batch;
   for (int ep = 0; ep < epochs; ++ep) {
     k_shuffle_idx<<<grid_for(ns, 256), 256, 0, r->stream>>>(idx, (int)ns, 0x5eedull + ep);
     RS_CUDA(cudaMemsetAsync(r->loss, 0, sizeof(float), r->stream));
     for (long bi = 0; bi < nbat; ++bi) {
-      RS_CUDA(cudaMemsetAsync(r->G, 0, NPARAM * sizeof(float), r->stream));
-      k_grad<<<(batch + TS - 1) / TS, TRAIN_THREADS, 0, r->stream>>>(r->w, d_x, d_t, idx + bi * batch, batch,
-                                                                      1.f / batch, r->G, r->loss);
+      k_grad<<<ctas, TRAIN_THREADS, sizeof(TrainSmem), r->stream>>>(r->w, d_x, d_t, idx + bi * batch, batch, 1.f / batch,
+                                                                   r->part);
       r->step++;
       float lr_ep = lr * powf(0.05f, (float)ep / (float)epochs);   // exponential decay to lr/20
-      k_adam<<<(NPARAM + 255) / 256, 256, 0, r->stream>>>(r->w, r->m, r->v, r->G, r->step, lr_ep, 0.9f, 0.999f, 1e-8f);
+      k_adam<<<RED_GRID, 256, 0, r->stream>>>(r->w, r->m, r->v, r->part, ctas, r->loss, r->step, lr_ep, 0.9f, 0.999f,
+                                              1e-8f);
     }
     float h = 0.f;
     RS_CUDA(cudaMemcpyAsync(&h, r->loss, sizeof(float), cudaMemcpyDeviceToHost, r->stream));
     RS_CUDA(cudaStreamSynchronize(r->stream));
     last = h / (float)(nbat * batch);
   }
-  cudaFree(idx);
   RS_CUDA(cudaGetLastError());
   if (loss_out) *loss_out = last;
   return repack(r);
