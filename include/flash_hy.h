@@ -357,10 +357,12 @@ int flash_hy_mark_refine_tree(flash_hy_ctx *ctx, int nvar, const int *vars, doub
 #define FLASH_HY_TUNE_MAX 8
 /* mx_runs: blocks a CTA of the mixed-precision 3D direction kernels
  * stages along the sweep -- 1, or FLASH_HY_MX_RUN where the context offers
- * runs (a full uniform grid of 8^3 blocks whose block counts divide by it,
- * no species): the CTA then takes runs of FLASH_HY_MX_RUN blocks and
- * 1/FLASH_HY_MX_RUN of their cross-section, which shares the stencil
- * overlap along the sweep.  The two are separately compiled FMA-contracted
+ * runs (a full uniform grid of 8^3 blocks whose block counts divide by it):
+ * the CTA then takes runs of FLASH_HY_MX_RUN blocks and a part of their
+ * cross-section (a quarter, or an eighth with HLLC, where it has at most
+ * 288 threads), which shares the stencil overlap along the sweep.  The FP64
+ * direction kernels take the same runs whatever is set: their results are
+ * bit-identical either way.  The two are separately compiled FMA-contracted
  * kernels, like the mx_threads candidates, and agree to rounding.  The
  * default is FLASH_HY_MX_RUN where offered; autotune tries both.        */
 #define FLASH_HY_MX_RUN 4
