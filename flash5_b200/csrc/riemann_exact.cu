@@ -729,6 +729,7 @@ struct flash_hy_rsolver {
   float *part;                  // k_grad's rows [GRAD_CTAS][PSTRIDE]
   int *idx;                     // train: the epoch's sample order
   long idx_cap;
+  int grad_set;                 // k_grad's shared-memory limit is raised
   unsigned *status;
   int step;
   int infer;                    // FLASH_HY_INFER_TCGEN05 or FLASH_HY_INFER_WARP_MMA
@@ -750,6 +751,15 @@ static int grid_for(long n, int threads) {
 
 constexpr long GRAD_CTAS = 296;         // two per SM
 static long grad_ctas(long nb) { const long t = (nb + TS - 1) / TS; return t < GRAD_CTAS ? t : GRAD_CTAS; }
+
+// k_grad's shared memory, raised on a solver's first use of it (loading the
+// kernel at create would cost every solver 0.7 ms)
+static int grad_ready(flash_hy_rsolver *r) {
+  if (r->grad_set) return 0;
+  RS_CUDA(cudaFuncSetAttribute(k_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem)));
+  r->grad_set = 1;
+  return 0;
+}
 
 static int repack(flash_hy_rsolver *r) {
   k_pack_mlp<<<1, 256, 0, r->stream>>>(r->w, r->packed);
@@ -828,7 +838,6 @@ extern "C" int flash_hy_rsolver_create(int device, flash_hy_rsolver **out) {
   r->tc_grid = sms * occ_s;
   r->tc_grid_p = sms * occ_p;
   r->infer = FLASH_HY_INFER_TCGEN05;
-  RS_CUDA(cudaFuncSetAttribute(k_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem)));
   return repack(r);
 }
 
@@ -927,6 +936,7 @@ extern "C" int flash_hy_rsolver_grad(flash_hy_rsolver *r, const float *d_x, cons
                                      float *h_grad, float *h_loss) {
   if (!r || !d_x || !d_t || !d_idx || nb <= 0) return FLASH_HY_ERR_BAD_ARG;
   RS_CUDA(cudaSetDevice(r->device));
+  if (int e = grad_ready(r)) return e;
   k_grad<<<(int)grad_ctas(nb), TRAIN_THREADS, sizeof(TrainSmem), r->stream>>>(r->w, d_x, d_t, d_idx, nb, 1.f / nb, r->part);
   k_reduce<<<RED_GRID, 256, 0, r->stream>>>(r->part, (int)grad_ctas(nb), r->G, r->loss);
   RS_CUDA(cudaGetLastError());
@@ -943,6 +953,7 @@ extern "C" int flash_hy_rsolver_train(flash_hy_rsolver *r, const float *d_x, con
                                       int batch, float lr, float *loss_out) {
   if (!r || !d_x || !d_t || ns < batch || batch <= 0 || epochs <= 0) return FLASH_HY_ERR_BAD_ARG;
   RS_CUDA(cudaSetDevice(r->device));
+  if (int e = grad_ready(r)) return e;
   if (r->idx_cap < ns) {
     if (r->idx) { RS_CUDA(cudaStreamSynchronize(r->stream)); cudaFree(r->idx); r->idx = nullptr; r->idx_cap = 0; }
     RS_CUDA(cudaMalloc((void **)&r->idx, ns * sizeof(int)));
