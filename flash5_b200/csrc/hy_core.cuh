@@ -149,7 +149,7 @@ template <> struct Arith<true> {
   bool bad = false;
   __device__ __forceinline__ void check(double x, bool when = true) {            // x = 0 or in range
     const unsigned u = (unsigned)__double2hiint(x) & 0x7fffffffu;
-    bad |= u - 0x20B00000u >= 0x3E800000u && u != 0u && when;
+    bad |= u - 0x20B00000u >= 0x3E800000u && (u | (unsigned)__double2loint(x)) != 0u && when;
   }
   __device__ __forceinline__ Rcp rcp(double b, bool when = true) {
     const unsigned hi = (unsigned)__double2hiint(b), u = hi & 0x7fffffffu;

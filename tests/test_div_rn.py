@@ -37,12 +37,18 @@ static void check(double x, double b) {
 /* Arith<true>: the seed keeps 20 bits of the reciprocal of b's leading 32 */
 static double seed(double b) { uint64_t u; memcpy(&u, &b, 8); u &= 0xFFFFFFFF00000000ull; memcpy(&b, &u, 8);
   double y = 1. / b; memcpy(&u, &y, 8); u &= 0xFFFFFFFF00000000ull; memcpy(&y, &u, 8); return y; }
-static int in_rng(double x) { uint64_t u; memcpy(&u, &x, 8); return ((uint32_t)(u >> 32) & 0x7fffffffu) - 0x20B00000u < 0x3E800000u; }
+/* the stated range: b and x (or x = 0) in [2^-500, 2^500), b's significand not all ones */
 static int refused(double x, double b) {
-  uint64_t u, v; memcpy(&u, &b, 8); memcpy(&v, &x, 8);
-  const uint32_t hi = (uint32_t)(u >> 32);
-  const int ones = ((hi | 0xfff00000u) & (uint32_t)u) == 0xffffffffu;
-  return !in_rng(b) || ones || (!in_rng(x) && ((uint32_t)(v >> 32) & 0x7fffffffu) != 0);
+  uint64_t u; memcpy(&u, &b, 8); u &= 0xFFFFFFFFFFFFFull;
+  return !(fabs(b) >= 0x1p-500 && fabs(b) < 0x1p500) || u == 0xFFFFFFFFFFFFFull ||
+         !(x == 0. || (fabs(x) >= 0x1p-500 && fabs(x) < 0x1p500));
+}
+/* the kernels' test of it (Arith<true>::check and rcp), on the words */
+static int bad_bits(double x, double b) {
+  uint64_t ub, ux; memcpy(&ub, &b, 8); memcpy(&ux, &x, 8);
+  const uint32_t hi = (uint32_t)(ub >> 32), v = (uint32_t)(ux >> 32) & 0x7fffffffu;
+  const int r = (hi & 0x7fffffffu) - 0x20B00000u >= 0x3E800000u || ((hi | 0xfff00000u) & (uint32_t)ub) == 0xffffffffu;
+  return r || (v - 0x20B00000u >= 0x3E800000u && (v | (uint32_t)ux) != 0u);
 }
 static double div_bf(double x, double b) {
   double y = seed(b);
@@ -53,7 +59,8 @@ static double div_bf(double x, double b) {
 }
 static void checkf(double x, double b) {
   double q = div_bf(x, b), r = x / b;
-  if (!refused(x, b) && memcmp(&q, &r, 8)) { if (bad < 5) printf("x=%a b=%a q=%a r=%a\n", x, b, q, r); ++bad; }
+  if (refused(x, b) != bad_bits(x, b)) { if (bad < 5) printf("range test: x=%a b=%a\n", x, b); ++bad; }
+  if (!bad_bits(x, b) && memcmp(&q, &r, 8)) { if (bad < 5) printf("x=%a b=%a q=%a r=%a\n", x, b, q, r); ++bad; }
 }
 int main(void) {
   const double cs[] = {3., 6.};
@@ -76,10 +83,14 @@ int main(void) {
   for (long i = 0; i < 3000000; ++i) { checkf(rnd(-60, 60), 3.); checkf(rnd(-60, 60), 6.); checkf(rnd(-60, 60), 12.); }
   const double z[] = {0., -0.};
   for (int i = 0; i < 2; ++i) { checkf(z[i], 3.); checkf(z[i], 0.7); }
-  const double out[] = {1e-310, 1e200, INFINITY, NAN, -1e-160};
-  for (int i = 0; i < 5; ++i) if (!refused(out[i], 1.5)) { printf("not refused %g\n", out[i]); ++bad; }
-  { uint64_t ones = 0x3FFFFFFFFFFFFFFFull; double b; memcpy(&b, &ones, 8); if (!refused(1., b)) ++bad; }
-  if (!refused(1., 0.) || !refused(1., 1e300)) ++bad;
+  const double out[] = {5e-324, -1e-315, 0x1p-1043, 1e-310, 1e200, INFINITY, NAN, -1e-160, 0x1.fp-501, 0x1p500};
+  for (int i = 0; i < 10; ++i) if (!refused(out[i], 1.5) || !bad_bits(out[i], 1.5)) { printf("not refused %g\n", out[i]); ++bad; }
+  for (long i = 0; i < 1000000; ++i) {           /* subnormal numerators */
+    uint64_t u = (nx() & 0xFFFFFFFFFFFFFull) >> (nx() % 52); double x; memcpy(&x, &u, 8);
+    checkf(nx() & 1 ? x : -x, i % 4 ? fabs(rnd(-40, 40)) : (i % 3 ? 6. : 12.));
+  }
+  { uint64_t ones = 0x3FFFFFFFFFFFFFFFull; double b; memcpy(&b, &ones, 8); if (!bad_bits(1., b)) ++bad; }
+  if (!bad_bits(1., 0.) || !bad_bits(1., 1e300) || !bad_bits(1., 0x1p500) || !bad_bits(1., 0x1.fp-501)) ++bad;
   printf("branch-free: mismatches %ld\n", bad - b0);
   printf("mismatches %ld\n", bad);
   return bad != 0;
