@@ -468,11 +468,14 @@ k_dir(const DevParams P, const double *__restrict__ SIG, double *__restrict__ AC
     sDb[6 * G::SB + q] = ft;
   };
   // (each phase runs with branch-free divisions; where any cell of the CTA
-  // needs plain ones, the CTA takes the phase again with those)
+  // needs plain ones, the CTA takes the phase again with those, and the
+  // status bits of the first attempt go)
   Arith<true> ar;
   Arith<false> plain;
+  unsigned st0 = st;
   for (int q = threadIdx.x; q < G::SB; q += blockDim.x) slopes(ar, q);
   if (__syncthreads_or(ar.bad)) {
+    st = st0;
     for (int q = threadIdx.x; q < G::SB; q += blockDim.x) slopes(plain, q);
     __syncthreads();
   }
@@ -581,8 +584,10 @@ k_dir(const DevParams P, const double *__restrict__ SIG, double *__restrict__ AC
     }
   };
   ar.bad = false;
+  st0 = st;
   for (int t = threadIdx.x; t < G::SC; t += blockDim.x) states(ar, t);
   if (__syncthreads_or(ar.bad)) {
+    st = st0;
     for (int t = threadIdx.x; t < G::SC; t += blockDim.x) states(plain, t);
     __syncthreads();
   }

@@ -317,8 +317,10 @@ __global__ void __launch_bounds__(320, NDIM > 2 ? (sizeof(R) == 4 ? 3 : 2) : 1) 
     Eig<R> eg;                               // one for the directions, which differ in the wave speeds only
     if constexpr (sizeof(R) == 8) {
       Arith<true> ar;
-      eigen64<1>(Vc, eg, ar, st);
-      if (ar.bad) { Arith<false> plain; eigen64<1>(Vc, eg, plain, st); }
+      unsigned se = 0;
+      eigen64<1>(Vc, eg, ar, se);
+      if (ar.bad) { Arith<false> plain; se = 0; eigen64<1>(Vc, eg, plain, se); }
+      st |= se;
     } else {
       R c[8];
 #pragma unroll
