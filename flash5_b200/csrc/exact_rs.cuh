@@ -41,12 +41,14 @@ struct MlpPacked {
 static_assert(sizeof(MlpPacked) % 16 == 0, "MlpPacked must be a multiple of 16 bytes");
 
 // ---------------------------------------------------------------------------
-// reciprocals and roots without branches: Newton's iteration (third order)
-// from the 20-bit seeds of rcp / rsqrt.approx.ftz.f64, the square root with
-// one residual correction.  Within an ulp for operands in [2^-500, 2^500)
-// (the seeds flush subnormals); the compiler's divisions and roots end their
-// basic block with a call for special operands, which keeps a solve's ten of
-// them from overlapping.
+// reciprocals, divisions and roots without branches: Newton's iteration
+// (third order) from the 20-bit seeds of rcp / rsqrt.approx.ftz.f64, its
+// residuals exact (FMA), divisions and square roots with one more residual
+// correction.  A result is one rounding of a value within 2^-60, relative:
+// within 0.51 ulp (tests/test_nr_arith.py).  For normal operands whose
+// products and residuals are normal too (the seeds flush subnormals).  The
+// compiler's divisions and roots end their basic block with a call for
+// special operands, which keeps a solve's ten of them from overlapping.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double rcp_nr(double b) {
   double y;
@@ -54,18 +56,25 @@ __device__ __forceinline__ double rcp_nr(double b) {
   const double e = fma(-b, y, 1.0);
   return fma(y, fma(e, e, e), y);
 }
-__device__ __forceinline__ double div_nr(double x, double b) {
-  const double y = rcp_nr(b), q = x * y;
+// x / b with y = rcp_nr(b)
+__device__ __forceinline__ double div_by(double x, double b, double y) {
+  const double q = x * y;
   return fma(fma(-q, b, x), y, q);
 }
+__device__ __forceinline__ double div_nr(double x, double b) { return div_by(x, b, rcp_nr(b)); }
+// (the product a y in two parts: its rounding would cost half an ulp)
 __device__ __forceinline__ double rsqrt_nr(double a) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(a));
-  const double e = fma(-(a * y), y, 1.0);
+  const double h = a * y, e = fma(-fma(a, y, -h), y, fma(-h, y, 1.0));
   return fma(y * e, fma(e, 0.375, 0.5), y);
 }
 __device__ __forceinline__ double sqrt_nr(double a) {
-  const double y = rsqrt_nr(a), q = a * y;
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(a));
+  const double e = fma(-(a * y), y, 1.0);
+  y = fma(y * e, fma(e, 0.375, 0.5), y);
+  const double q = a * y;
   return fma(0.5 * y, fma(-q, q, a), q);
 }
 // whether x > 0 lies in [2^-300, 2^300): operands in that range keep the
@@ -146,7 +155,6 @@ __device__ __forceinline__ double pow_n_d(double w, const PowN &e, double &dpdw)
 // two-rarefaction guess and the sampling (section 4.5).
 struct Gas {
   double g, z, gm1inv, k2, a2, g6, g2, hgm1;   // 1/(g-1), 2/(g-1), 2/(g+1), (g-1)/(g+1), (g+1)/(2g), (g-1)/2
-  double s0;                                   // sqrt(2/((g+1) g)): sqrt(A_K p_K) = s0 c_K
   PowN e;
 };
 __host__ __device__ __forceinline__ Gas gas_of(double g) {
@@ -159,24 +167,23 @@ __host__ __device__ __forceinline__ Gas gas_of(double g) {
   s.g6 = (g - 1.0) / (g + 1.0);
   s.g2 = (g + 1.0) / (2.0 * g);
   s.hgm1 = 0.5 * (g - 1.0);
-  s.s0 = sqrt(s.a2 / g);
   s.e = pown_of(2.0 * g / (g - 1.0));
   return s;
 }
 // the same without branches, for a gas per solve
 __device__ __forceinline__ Gas gas_nr(double g) {
   Gas s;
-  const double gm1 = g - 1.0, r1 = rcp_nr(gm1), r2 = rcp_nr(g + 1.0);
+  const double gm1 = g - 1.0, gp1 = g + 1.0, tg = 2.0 * g;
+  const double r1 = rcp_nr(gm1), r2 = rcp_nr(gp1), r3 = rcp_nr(tg);
   s.g = g;
-  s.z = div_nr(gm1, 2.0 * g);
+  s.z = div_by(gm1, tg, r3);
   s.gm1inv = r1;
   s.k2 = 2.0 * r1;
   s.a2 = 2.0 * r2;
-  s.g6 = gm1 * r2;
-  s.g2 = 1.0 - s.z;
+  s.g6 = div_by(gm1, gp1, r2);
+  s.g2 = div_by(gp1, tg, r3);
   s.hgm1 = 0.5 * gm1;
-  s.s0 = sqrt_nr(div_nr(s.a2, g));
-  s.e = pown_of(2.0 * g * r1);
+  s.e = pown_of(div_by(tg, gm1, r1));
   return s;
 }
 
@@ -187,27 +194,44 @@ __device__ __forceinline__ double p_of_w(double w, const Gas &G) { return pow_n(
 // p_K / p_L, the rarefaction slope k = 2 c_K / ((g-1) w_K), s = sqrt(A_K
 // p_L) and B_K / p_L of the shock branch.
 struct SideK { double w, P, k, s, B; };
-// sound speeds of a pair (d, u, p given); the branch-free roots hold over
-// [2^-300, 2^300), others take the compiler's
-__device__ __forceinline__ bool sound(Side &L, Side &R, const Gas &G) {
-  const bool fast = in_range(L.d) && in_range(L.p) && in_range(R.d) && in_range(R.p);
-  if (fast) {
-    L.c = sqrt_nr(G.g * L.p * rcp_nr(L.d));
-    R.c = sqrt_nr(G.g * R.p * rcp_nr(R.d));
+// whether the branch-free arithmetic holds for a pair: densities and
+// pressures in [2^-300, 2^300)
+__device__ __forceinline__ bool fast_pair(const Side &L, const Side &R) {
+  return in_range(L.d) && in_range(L.p) && in_range(R.d) && in_range(R.p);
+}
+// sound speeds of a pair (d, u, p given)
+__device__ __forceinline__ void sound(Side &L, Side &R, const Gas &G) {
+  if (fast_pair(L, R)) {
+    L.c = sqrt_nr(div_nr(G.g * L.p, L.d));
+    R.c = sqrt_nr(div_nr(G.g * R.p, R.d));
   } else {
     L.c = sqrt(G.g * L.p / L.d);
     R.c = sqrt(G.g * R.p / R.d);
   }
-  return fast;
 }
-// and w and the pressure functions
+// and w and the pressure functions (s from the densities and pressures, not
+// from the sound speeds, whose roundings would add to it)
 __device__ __forceinline__ void setup(Side &L, Side &R, const Gas &G, SideK &kl, SideK &kr) {
-  const bool fast = sound(L, R, G);
-  const double x = fast ? div_nr(R.p, L.p) : R.p / L.p;
+  double x, sl, sr;
+  const double a = G.a2 * L.p;
+  if (fast_pair(L, R)) {
+    const double yl = rcp_nr(L.d), yr = rcp_nr(R.d);
+    L.c = sqrt_nr(div_by(G.g * L.p, L.d, yl));
+    R.c = sqrt_nr(div_by(G.g * R.p, R.d, yr));
+    sl = sqrt_nr(div_by(a, L.d, yl));
+    sr = sqrt_nr(div_by(a, R.d, yr));
+    x = div_nr(R.p, L.p);
+  } else {
+    L.c = sqrt(G.g * L.p / L.d);
+    R.c = sqrt(G.g * R.p / R.d);
+    sl = sqrt(a / L.d);
+    sr = sqrt(a / R.d);
+    x = R.p / L.p;
+  }
   L.w = 1.0;
   R.w = powp(x, G.z);
-  kl = SideK{1.0, 1.0, G.k2 * L.c, G.s0 * L.c, G.g6};
-  kr = SideK{R.w, x, G.k2 * R.c * rcp_nr(R.w), G.s0 * R.c * rsqrt_nr(x), G.g6 * x};
+  kl = SideK{1.0, 1.0, G.k2 * L.c, sl, G.g6};
+  kr = SideK{R.w, x, div_nr(G.k2 * R.c, R.w), sr, G.g6 * x};
 }
 
 // f_K(w) and df_K/dw (Toro eqs. 4.6-4.7 with P = w^n, dP/dw = dpdw): both

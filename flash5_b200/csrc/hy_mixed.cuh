@@ -84,10 +84,10 @@ __device__ __forceinline__ bool hllc_fp64(const DevParams &P, const double *Vm, 
   const int lo = max(__double2hiint(P.tiny), 0x2D300000);          // tiny or 2^-300
   const bool ok = at_least(dL, lo) && at_least(dR, lo) && at_least(pL, lo) && at_least(pR, lo);
   const double rL = xrs::rcp_nr(dL), rR = xrs::rcp_nr(dR);
-  const double cL = xrs::sqrt_nr(P.gamma * pL * rL), cR = xrs::sqrt_nr(P.gamma * pR * rR);
+  const double cL = xrs::sqrt_nr(xrs::div_by(P.gamma * pL, dL, rL)), cR = xrs::sqrt_nr(xrs::div_by(P.gamma * pR, dR, rR));
   const double SL = fmin(uL - cL, uR - cR), SR = fmax(uL + cL, uR + cR);
   const double mL = __dmul_rn(dL, SL - uL), mR = __dmul_rn(dR, SR - uR);
-  const double qStar = (fma(uR, mR, -__dmul_rn(uL, mL)) + (pL - pR)) * xrs::rcp_nr(__dsub_rn(mR, mL));
+  const double qStar = xrs::div_nr(fma(uR, mR, -__dmul_rn(uL, mL)) + (pL - pR), __dsub_rn(mR, mL));
   const double pStar = fma(mL, qStar - uL, pL);
   // side whose flux (and star state) is used
   const bool useL = SL >= 0. || qStar >= 0.;
@@ -105,7 +105,7 @@ __device__ __forceinline__ bool hllc_fp64(const DevParams &P, const double *Vm, 
   Fs[DIR] = star ? fma(g, fma(r1, qStar, qStar - u), fn) : fn;
   Fs[4] = star ? fma(S, fma(E, r1, __dmul_rn(fma(pStar, qStar, -__dmul_rn(p, u)), rden)), fe) : fe;
   Fs[5] = p;
-  fv = a * (a > 0. ? rL : rR);
+  fv = xrs::div_by(a, a > 0. ? dL : dR, a > 0. ? rL : rR);
   return ok;
 }
 
@@ -922,7 +922,7 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
           pb = (0.5 * sx) * 0.5 + sp * 0.25;
         } else {
           const double sy = AUX[5 * ncells + off];
-          pb = (((0.5 * sx) * 0.5 + sy * 0.25) * 4.0 + sp) * (1.0 / 6.0);
+          pb = xrs::div_by(((0.5 * sx) * 0.5 + sy * 0.25) * 4.0 + sp, 6.0, 1.0 / 6.0);
         }
         IntEner = rho0 * e0 + dt / del[0] * (AUX[off] + pb * AUX[ncells + off]);
         if (NDIM == 2) {
@@ -943,7 +943,7 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
         }
         double pb;
         if (NDIM == 2) pb = (0.5 * ts[0]) * 0.5 + ts[1] * 0.25;
-        else pb = (((0.5 * ts[0]) * 0.5 + ts[1] * 0.25) * 4.0 + ts[2]) * (1.0 / 6.0);
+        else pb = xrs::div_by(((0.5 * ts[0]) * 0.5 + ts[1] * 0.25) * 4.0 + ts[2], 6.0, 1.0 / 6.0);
         IntEner = rho0 * e0 + dt / del[0] * (te[0] + pb * tb[0]);
         IntEner += dt / del[1] * (te[1] + pb * tb[1]);
         if (NDIM == 3) IntEner += dt / del[2] * (te[2] + pb * tb[2]);
