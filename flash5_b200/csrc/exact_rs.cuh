@@ -194,44 +194,33 @@ __device__ __forceinline__ double p_of_w(double w, const Gas &G) { return pow_n(
 // p_K / p_L, the rarefaction slope k = 2 c_K / ((g-1) w_K), s = sqrt(A_K
 // p_L) and B_K / p_L of the shock branch.
 struct SideK { double w, P, k, s, B; };
-// whether the branch-free arithmetic holds for a pair: densities and
-// pressures in [2^-300, 2^300)
+// Whether the branch-free arithmetic holds for a pair: densities and
+// pressures in [2^-300, 2^300), so that ratios and their powers stay normal
+// too.  sound, setup and what follows from them are of no use for other
+// pairs; those go through solve_any.
 __device__ __forceinline__ bool fast_pair(const Side &L, const Side &R) {
   return in_range(L.d) && in_range(L.p) && in_range(R.d) && in_range(R.p);
 }
 // sound speeds of a pair (d, u, p given)
 __device__ __forceinline__ void sound(Side &L, Side &R, const Gas &G) {
-  if (fast_pair(L, R)) {
-    L.c = sqrt_nr(div_nr(G.g * L.p, L.d));
-    R.c = sqrt_nr(div_nr(G.g * R.p, R.d));
-  } else {
-    L.c = sqrt(G.g * L.p / L.d);
-    R.c = sqrt(G.g * R.p / R.d);
-  }
+  L.c = sqrt_nr(div_nr(G.g * L.p, L.d));
+  R.c = sqrt_nr(div_nr(G.g * R.p, R.d));
 }
 // and w and the pressure functions (s from the densities and pressures, not
-// from the sound speeds, whose roundings would add to it)
+// from the sound speeds, whose roundings would add to it).  TEST: behind a
+// branch on fast_pair, which keeps k_solve_tc from spilling (15M learned
+// solves 1.19 ms; without it 1.22; the two-rarefaction kernel is faster
+// without, 4.43 against 4.47 ms for 1e8).
+template <bool TEST = false>
 __device__ __forceinline__ void setup(Side &L, Side &R, const Gas &G, SideK &kl, SideK &kr) {
-  double x, sl, sr;
-  const double a = G.a2 * L.p;
-  if (fast_pair(L, R)) {
-    const double yl = rcp_nr(L.d), yr = rcp_nr(R.d);
-    L.c = sqrt_nr(div_by(G.g * L.p, L.d, yl));
-    R.c = sqrt_nr(div_by(G.g * R.p, R.d, yr));
-    sl = sqrt_nr(div_by(a, L.d, yl));
-    sr = sqrt_nr(div_by(a, R.d, yr));
-    x = div_nr(R.p, L.p);
-  } else {
-    L.c = sqrt(G.g * L.p / L.d);
-    R.c = sqrt(G.g * R.p / R.d);
-    sl = sqrt(a / L.d);
-    sr = sqrt(a / R.d);
-    x = R.p / L.p;
-  }
+  if (TEST && !fast_pair(L, R)) return;
+  const double yl = rcp_nr(L.d), yr = rcp_nr(R.d), a = G.a2 * L.p, x = div_nr(R.p, L.p);
+  L.c = sqrt_nr(div_by(G.g * L.p, L.d, yl));
+  R.c = sqrt_nr(div_by(G.g * R.p, R.d, yr));
   L.w = 1.0;
   R.w = powp(x, G.z);
-  kl = SideK{1.0, 1.0, G.k2 * L.c, sl, G.g6};
-  kr = SideK{R.w, x, div_nr(G.k2 * R.c, R.w), sr, G.g6 * x};
+  kl = SideK{1.0, 1.0, G.k2 * L.c, sqrt_nr(div_by(a, L.d, yl)), G.g6};
+  kr = SideK{R.w, x, div_nr(G.k2 * R.c, R.w), sqrt_nr(div_by(a, R.d, yr)), G.g6 * x};
 }
 
 // f_K(w) and df_K/dw (Toro eqs. 4.6-4.7 with P = w^n, dP/dw = dpdw): both
@@ -300,13 +289,15 @@ struct Star { double p, u, w; };
 // Newton on f(w) = f_L + f_R + (u_R - u_L) from w0 >= 0.  Converged when
 // the step is below tol * z * w (a relative step of tol in p); once the
 // last two steps show the quadratic regime, when the predicted next step
-// |step|^3 / prev^2 is below a hundredth of that; or when the bracket
+// |step|^3 / prev^2 is below a hundredth of that (WIDE: asked of w in
+// [2^-300, 2^300), where the products stay in range); or when the bracket
 // [wa, wb] of evaluated signs is that narrow (near vacuum, where the
 // rounding of f exceeds the tolerance on the step; the root is its
 // midpoint).  A step that leaves the bracket is replaced by its midpoint
 // (or a doubling while no upper end is known).  u* is f_L, f_R linearised
 // from the last evaluation to the returned w*.  Returns the number of
 // evaluations, or -max_iter when not converged.
+template <bool WIDE = false>
 __device__ __forceinline__ int newton(const Side &L, const Side &R, const SideK &kl, const SideK &kr, const Gas &G,
                                       double w0, double tol, int max_iter, Star &out) {
   const double du = R.u - L.u, ztol = G.z * tol;
@@ -332,7 +323,7 @@ __device__ __forceinline__ int newton(const Side &L, const Side &R, const SideK 
     const bool narrow = wb - wa <= ztol * w, inside = wn > wa && wn < wb;
     // f == 0: the root; a narrow bracket: its midpoint; else the step
     done = f == 0.0 || narrow || as <= ztol * w ||
-           (inside && prev > 0.0 && as < prev && as * as * as <= 0.01 * ztol * w * (prev * prev));
+           (inside && prev > 0.0 && as < prev && (!WIDE || in_range(w)) && as * as * as <= 0.01 * ztol * w * (prev * prev));
     wend = f == 0.0 ? w : (narrow ? 0.5 * (wa + wb) : (wn > 0.0 ? wn : w));
     if (!inside) {
       wn = wb == DBL_MAX ? 2.0 * w : 0.5 * (wa + wb);
@@ -396,16 +387,48 @@ __device__ __forceinline__ void sample0(const Side &L, const Side &R, const Gas 
   if (right) u = -u;
 }
 
-// Godunov flux of the exact solution in the 6-slot layout of the HLLC
-// solver (mass, three momenta, energy, pressure).  VL, VR are primitive
-// states in the slot order dens, velx, vely, velz, pres, ...; DIR is the
-// normal direction (1..3).
+// The solve and the sampling of a pair out of the range of the branch-free
+// arithmetic (fast_pair), whose pressures may be 2^1000 apart: pressures
+// relative to a power of two halfway between them, so that they and the
+// iteration stay normal, the compiler's divisions and roots in the set-up.
+// Not inlined: pairs in the range pay a test for it.
+struct AnyPair { double d, u, p, ps, us; int k; bool vac, right; };   // state at x/t = 0, star state, newton's count
+static __device__ __noinline__ void solve_any(const Side *left, const Side *rght, double g, double tol, int max_iter,
+                                              AnyPair *out) {
+  const Gas G = gas_of(g);
+  Side L = *left, R = *rght;
+  const bool pos = L.p > 0.0 && L.p <= DBL_MAX && R.p > 0.0 && R.p <= DBL_MAX;
+  const double p0 = pos ? scalbn(1.0, (ilogb(L.p) + ilogb(R.p)) / 2) : 1.0, sp = sqrt(p0);
+  L.c = sqrt(g * L.p / L.d);
+  R.c = sqrt(g * R.p / R.d);
+  L.p = L.p / p0;
+  R.p = R.p / p0;
+  L.w = powp(L.p, G.z);
+  R.w = powp(R.p, G.z);
+  const SideK kl{L.w, L.p, G.k2 * L.c / L.w, sqrt(G.a2 / L.d) * sp, G.g6 * L.p};
+  const SideK kr{R.w, R.p, G.k2 * R.c / R.w, sqrt(G.a2 / R.d) * sp, G.g6 * R.p};
+  Star S{0.0, 0.5 * (L.u + R.u), 0.0};
+  out->vac = vacuum(L, R, G);
+  out->k = 0;
+  if (!out->vac) {
+    const double num = L.c + R.c - G.hgm1 * (R.u - L.u);
+    Side one = L;
+    one.p = 1.0;                                     // what newton's P is relative to
+    out->k = newton<true>(one, R, kl, kr, G, num > 0.0 ? num / (G.hgm1 * (kl.k + kr.k)) : 0.0, tol, max_iter, S);
+  }
+  sample0(L, R, G, S, out->vac, out->d, out->u, out->p, out->right);
+  out->p *= p0;
+  out->ps = S.p * p0;
+  out->us = S.u;
+}
+
+// Godunov flux of the state (d, u, p) at x/t = 0, the transverse velocities
+// from its side, in the 6-slot layout of the HLLC solver (mass, three
+// momenta, energy, pressure).  VL, VR are primitive states in the slot order
+// dens, velx, vely, velz, pres, ...; DIR is the normal direction (1..3).
 template <int DIR>
-__device__ __forceinline__ void godunov_flux(const double *VL, const double *VR, const Side &L, const Side &R,
-                                             const Gas &G, const Star &S, bool vac, double F[6]) {
-  double d, u, p;
-  bool right;
-  sample0(L, R, G, S, vac, d, u, p, right);
+__device__ __forceinline__ void godunov_flux(const double *VL, const double *VR, const Gas &G, double d, double u,
+                                             double p, bool right, double F[6]) {
   double v[3];
 #pragma unroll
   for (int m = 0; m < 3; ++m) v[m] = (m == DIR - 1) ? u : (right ? VR[1 + m] : VL[1 + m]);

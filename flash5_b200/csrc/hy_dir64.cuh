@@ -592,8 +592,10 @@ k_dir(const DevParams P, const double *__restrict__ SIG, double *__restrict__ AC
     __syncthreads();
   }
 
-  // ---- faces
-  auto faces = [&](auto &ar, int t) {
+  // ---- faces (exact solver: again, the pairs out of its range alone, after
+  // the loop, so that it holds no call)
+  bool redo = false;
+  auto faces = [&](auto &ar, int t, auto again) {
     int x, l;
     G::dec(t, G::LC, 1, x, l);
     if (x < 0) return;
@@ -605,9 +607,13 @@ k_dir(const DevParams P, const double *__restrict__ SIG, double *__restrict__ AC
     }
     VL[HGE] = sGe[t - G::step]; VR[HGE] = sGe[t];
     VL[HGC] = P.gamma; VR[HGC] = P.gamma;
+    if constexpr (decltype(again)::value) {
+      if (xrs::fast_pair(xrs::Side{VL[HD], 0., VL[HP]}, xrs::Side{VR[HD], 0., VR[HP]})) return;
+    }
     double F[6], fv, fe;
     if constexpr (RS == 1) {
-      exact_face<DIR>(P, P.gas, VL, VR, F, st);
+      if constexpr (decltype(again)::value) exact_face_any<DIR>(P, P.gas, VL, VR, F, st);
+      else redo |= exact_face<DIR>(P, P.gas, VL, VR, F, st);
       fv = F[FDENS] / (F[FDENS] > 0. ? VL[HD] : VR[HD]);
     } else {
       hllc64<DIR>(P, ar, VL, VR, F, fv, st);
@@ -622,9 +628,13 @@ k_dir(const DevParams P, const double *__restrict__ SIG, double *__restrict__ AC
       seam_blocks<K, G::N0, true>(x, [&](int m, int y) { P.sp_mf[sp_line(m, y, l)] = F[FDENS]; });
   };
   ar.bad = false;
-  for (int t = threadIdx.x; t < G::SC; t += blockDim.x) faces(ar, t);
+  for (int t = threadIdx.x; t < G::SC; t += blockDim.x) faces(ar, t, std::false_type());
+  if constexpr (RS == 1) {
+    if (redo)
+      for (int t = threadIdx.x; t < G::SC; t += blockDim.x) faces(ar, t, std::true_type());
+  }
   if (__syncthreads_or(ar.bad)) {
-    for (int t = threadIdx.x; t < G::SC; t += blockDim.x) faces(plain, t);
+    for (int t = threadIdx.x; t < G::SC; t += blockDim.x) faces(plain, t, std::false_type());
     __syncthreads();
   }
   if (K == 1 && P.freg) {       // AMR: fine/coarse faces

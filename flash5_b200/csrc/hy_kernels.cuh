@@ -488,17 +488,33 @@ __device__ __forceinline__ void harvest_face(const DevParams &P, const xrs::Side
   S[3 * c + k] = R.d; S[4 * c + k] = R.u; S[5 * c + k] = R.p; S[6 * c + k] = g;
 }
 
-// Godunov flux from the exact solution, Newton from the two-rarefaction guess
+// Godunov flux from the exact solution, Newton from the two-rarefaction
+// guess; true for a pair out of the range of the branch-free arithmetic,
+// whose flux is left to exact_face_any
 template <int DIR>
-__device__ __forceinline__ void exact_face(const DevParams &P, const xrs::Gas &G, const double *VL, const double *VR,
+__device__ __forceinline__ bool exact_face(const DevParams &P, const xrs::Gas &G, const double *VL, const double *VR,
                                            double F[6], unsigned &st) {
   xrs::Side L = side_of(VL[HD], VL[DIR], VL[HP], st), R = side_of(VR[HD], VR[DIR], VR[HP], st);
   xrs::SideK kl, kr;
   xrs::setup(L, R, G, kl, kr);
-  const bool vac = xrs::vacuum(L, R, G);
+  const bool any = !xrs::fast_pair(L, R), vac = any || xrs::vacuum(L, R, G);
   xrs::Star S{0.0, 0.5 * (L.u + R.u), 0.0};
   if (!vac && xrs::newton(L, R, kl, kr, G, xrs::tr_w(L, R, kl, kr, G), P.rs_tol, P.rs_max_iter, S) < 0) st |= ST_NEWTON;
-  xrs::godunov_flux<DIR>(VL, VR, L, R, G, S, vac, F);
+  double d, u, p;
+  bool right;
+  xrs::sample0(L, R, G, S, vac, d, u, p, right);
+  xrs::godunov_flux<DIR>(VL, VR, G, d, u, p, right, F);
+  return any;
+}
+template <int DIR>
+__device__ __forceinline__ void exact_face_any(const DevParams &P, const xrs::Gas &G, const double *VL,
+                                               const double *VR, double F[6], unsigned &st) {
+  unsigned seen = 0;                              // exact_face has reported the sides
+  const xrs::Side L = side_of(VL[HD], VL[DIR], VL[HP], seen), R = side_of(VR[HD], VR[DIR], VR[HP], seen);
+  xrs::AnyPair a;
+  xrs::solve_any(&L, &R, G.g, P.rs_tol, P.rs_max_iter, &a);
+  if (a.k < 0) st |= ST_NEWTON;
+  xrs::godunov_flux<DIR>(VL, VR, G, a.d, a.u, a.p, a.right, F);
 }
 
 // ---------------------------------------------------------------------------

@@ -669,7 +669,9 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
       return left ? Vs(qq, s.y) + double(sWp[qq * G::SC + t - G::step])
                   : Vs(qq, s.x) + double(sWm[qq * G::SC + t]);
     };
-    // the two face states (sound speeds and the rest by xrs::sound / setup)
+    // the two face states (sound speeds and the rest by xrs::sound / setup;
+    // densities and pressures out of xrs::fast_pair's range are far out of
+    // that of the FP32 reconstruction: such a state arrives as NaN)
     auto sides = [&](int2 s, int t, xrs::Side &L, xrs::Side &R) {
       L = side_of(face(0, true, s, t), face(DIR, true, s, t), face(4, true, s, t), st);
       R = side_of(face(0, false, s, t), face(DIR, false, s, t), face(4, false, s, t), st);
@@ -777,7 +779,10 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
         VR[n] = face(qq, false, s, t);
       }
       double F[9];
-      xrs::godunov_flux<DIR>(VL, VR, L, R, gas, S, vac, F);
+      double d, u, p;
+      bool right;
+      xrs::sample0(L, R, gas, S, vac, d, u, p, right);
+      xrs::godunov_flux<DIR>(VL, VR, gas, d, u, p, right, F);
       double fv = 0., fe = 0.;
       if (P.use_aux_eint) {
         const bool up = F[FDENS] > 0.;

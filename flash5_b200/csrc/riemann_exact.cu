@@ -37,27 +37,33 @@ using namespace xrs;
 // ---------------------------------------------------------------------------
 constexpr int SOLVE_THREADS = 256;
 
-__device__ __forceinline__ void load_state(const double *__restrict__ S, long n, long i, Side &L, Side &R, Gas &G,
+// the state of pair i; true for a pair out of the range of the branch-free
+// arithmetic
+template <bool TEST = false>
+__device__ __forceinline__ bool load_state(const double *__restrict__ S, long n, long i, Side &L, Side &R, Gas &G,
                                            SideK &kl, SideK &kr) {
   L.d = S[i]; L.u = S[n + i]; L.p = S[2 * n + i];
   R.d = S[3 * n + i]; R.u = S[4 * n + i]; R.p = S[5 * n + i];
+  const bool any = !fast_pair(L, R);
   G = gas_nr(S[6 * n + i]);
-  setup(L, R, G, kl, kr);
+  setup<TEST>(L, R, G, kl, kr);
+  return any;
 }
 
 // the state of pair i, or that of the last pair for a lane past the end
 // (lanes of the last tile take part in the warp and CTA collectives)
-__device__ __forceinline__ void load_or_last(const double *__restrict__ S, long n, long i, Side &L, Side &R, Gas &G,
+template <bool TEST = false>
+__device__ __forceinline__ bool load_or_last(const double *__restrict__ S, long n, long i, Side &L, Side &R, Gas &G,
                                              SideK &kl, SideK &kr) {
-  load_state(S, n, i < n ? i : n - 1, L, R, G, kl, kr);
+  return load_state<TEST>(S, n, i < n ? i : n - 1, L, R, G, kl, kr);
 }
 
 // Newton from w0 (three evaluations where the network gave the start, else
 // max_iter) and the recording of the result; returns true where a network
 // start did not converge, so that the pair is queued for k_fallback
 __device__ __forceinline__ bool solve_store(const Side &L, const Side &R, const SideK &kl, const SideK &kr,
-                                            const Gas &G, bool vac, bool net, double w0, double tol, int max_iter,
-                                            bool valid, long i, long n, double *__restrict__ out,
+                                            const Gas &G, bool vac, bool net, double w0, double tol,
+                                            int max_iter, bool valid, long i, long n, double *__restrict__ out,
                                             unsigned char *__restrict__ iters, unsigned char *__restrict__ flags,
                                             unsigned &st) {
   unsigned char fl = net ? 8 : 0;
@@ -78,6 +84,22 @@ __device__ __forceinline__ bool solve_store(const Side &L, const Side &R, const 
     if (flags) flags[i] = fl;
   }
   return pending;
+}
+
+// Pair i where it is out of the range of the branch-free arithmetic, from
+// the two-rarefaction start (the network's FP32 features cannot hold it).
+__device__ __forceinline__ void solve_store_any(const double *__restrict__ S, long n, long i, double tol, int max_iter,
+                                                double *__restrict__ out, unsigned char *__restrict__ iters,
+                                                unsigned char *__restrict__ flags, unsigned &st) {
+  const Side L{S[i], S[n + i], S[2 * n + i]}, R{S[3 * n + i], S[4 * n + i], S[5 * n + i]};
+  if (fast_pair(L, R)) return;
+  AnyPair a;
+  solve_any(&L, &R, S[6 * n + i], tol, max_iter, &a);
+  const int its = a.k < 0 ? max_iter : a.k;
+  out[i] = a.ps; out[n + i] = a.us;
+  if (iters) iters[i] = (unsigned char)(its > 255 ? 255 : its);
+  if (flags) flags[i] = a.vac ? 2 : (a.k < 0 ? 4 : 0);
+  if (a.k < 0) st |= FLASH_HY_ERR_NEWTON_NOCONV;
 }
 
 // append the warp's pending lanes to the fallback queue (one atomic per warp)
@@ -102,8 +124,10 @@ __device__ __forceinline__ void enqueue(bool pending, long i, int *queue, int *q
 // One instantiation per path, so that the two-rarefaction path does not
 // carry the network's register footprint.  Bound by FP64 issue and latency;
 // 1e8 pairs on B200, two-rarefaction start: 8.84 ms with two powers, IEEE
-// divisions and roots per solve (16 warps per SM) -> 4.33 ms with one power
-// and branch-free arithmetic (exact_rs.cuh), 4.24 at 64 registers (32 warps).
+// divisions and roots per solve (16 warps per SM) -> 4.43 ms with one power
+// and branch-free arithmetic (exact_rs.cuh) at 64 registers (32 warps).
+// Pairs out of that arithmetic's range follow after the loop, which then
+// holds no call; the learned forms queue them for k_fallback.
 template <bool learned>
 __global__ void __launch_bounds__(SOLVE_THREADS, learned ? 2 : 4)
 k_solve(const double *__restrict__ S, long n, double *__restrict__ out, unsigned char *__restrict__ iters,
@@ -113,6 +137,7 @@ k_solve(const double *__restrict__ S, long n, double *__restrict__ out, unsigned
   if (learned) { load_packed(M, w); __syncthreads(); }
   const long stride = (long)gridDim.x * blockDim.x;
   unsigned st = 0;
+  bool redo = false;
   // grid-stride loop whose trip count is uniform across a warp
   for (long base = (long)blockIdx.x * blockDim.x; base < n; base += stride) {
     const long i = base + threadIdx.x;
@@ -120,8 +145,8 @@ k_solve(const double *__restrict__ S, long n, double *__restrict__ out, unsigned
     Side L, R;
     Gas G;
     SideK kl, kr;
-    load_or_last(S, n, i, L, R, G, kl, kr);
-    const bool vac = vacuum(L, R, G);
+    const bool any = load_or_last(S, n, i, L, R, G, kl, kr), vac = any || vacuum(L, R, G);
+    if (!learned) redo |= any;
     const double wtr = vac ? 0.0 : tr_w(L, R, kl, kr, G);
     const double ptr = vac ? 0.0 : L.p * p_of_w(wtr, G);
     double w0 = wtr;
@@ -139,8 +164,11 @@ k_solve(const double *__restrict__ S, long n, double *__restrict__ out, unsigned
       }
     }
     const bool pending = solve_store(L, R, kl, kr, G, vac, net, w0, tol, max_iter, valid, i, n, out, iters, flags, st);
-    if (learned) enqueue(pending && valid, i, queue, qcount);
+    if (learned) enqueue((pending || any) && valid, i, queue, qcount);
   }
+  if (!learned && redo)
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+      solve_store_any(S, n, i, tol, max_iter, out, iters, flags, st);
   if (st) atomicOr(status, st);
 }
 
@@ -266,8 +294,7 @@ k_solve_tc(const double *__restrict__ S, long n, double *__restrict__ out, unsig
     Side L, R;
     Gas G;
     SideK kl, kr;
-    load_or_last(S, n, i, L, R, G, kl, kr);
-    const bool vac = vacuum(L, R, G);
+    const bool any = load_or_last<true>(S, n, i, L, R, G, kl, kr), vac = any || vacuum(L, R, G);
     const double wtr = vac ? 0.0 : tr_w(L, R, kl, kr, G);
     const double ptr = vac ? 0.0 : L.p * p_of_w(wtr, G);
     const bool net = SOLVE ? (valid && !vac && !tr_exact(L, R, ptr) && strong_waves(L, R)) : (valid && !vac);
@@ -284,9 +311,9 @@ k_solve_tc(const double *__restrict__ S, long n, double *__restrict__ out, unsig
     }
     tc05::fence_smem_to_async();
     tc05::fence_before_sync();
-    const bool any = __syncthreads_or(net);
+    const bool consult = __syncthreads_or(net);
     if (sm.fail) { bail = true; break; }
-    if (any) {
+    if (consult) {
       if (t == 0) {
         tc05::fence_after_sync();
         tc05::mma_bf16(tmem, tc05::sdesc(xs, kLbo, kSboA1), tc05::sdesc(w1s, kLbo, kSboA1), idesc64, 0u);
@@ -362,7 +389,7 @@ k_solve_tc(const double *__restrict__ S, long n, double *__restrict__ out, unsig
       if (net) w0 = wtr * (double)expf(float(G.z) * fminf(fmaxf(y, -20.f), 20.f));   // (p*/p_TR)^z
       const bool pending = solve_store(L, R, kl, kr, G, vac, net, w0, tol, max_iter, valid, i, n, out, iters,
                                        flags, st);
-      enqueue(pending && valid, i, queue, qcount);
+      enqueue((pending || any) && valid, i, queue, qcount);
     } else if (valid) {
       yout[i] = net ? y : 0.f;
     }
@@ -382,7 +409,8 @@ k_solve_tc(const double *__restrict__ S, long n, double *__restrict__ out, unsig
   }
 }
 
-// fallback: queued solves restart from the two-rarefaction guess
+// fallback: queued solves restart from the two-rarefaction guess; pairs out
+// of the range of the branch-free arithmetic
 __global__ void __launch_bounds__(SOLVE_THREADS) k_fallback(const double *__restrict__ S, long n,
                                                             double *__restrict__ out, unsigned char *__restrict__ iters,
                                                             unsigned char *__restrict__ flags, const int *queue,
@@ -395,7 +423,10 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_fallback(const double *__rest
     Side L, R;
     Gas G;
     SideK kl, kr;
-    load_state(S, n, i, L, R, G, kl, kr);
+    if (load_state(S, n, i, L, R, G, kl, kr)) {
+      solve_store_any(S, n, i, tol, max_iter, out, iters, flags, st);
+      continue;
+    }
     Star S;
     unsigned char fl = 1 | 8;
     int k = newton(L, R, kl, kr, G, tr_w(L, R, kl, kr, G), tol, max_iter, S);
@@ -408,7 +439,8 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_fallback(const double *__rest
   if (st) atomicOr(status, st);
 }
 
-// network output y = MLP(features) for every interface (0 for vacuum cases)
+// network output y = MLP(features) for every interface (0 for vacuum cases
+// and for pairs whose densities or pressures its FP32 features cannot hold)
 __global__ void __launch_bounds__(SOLVE_THREADS) k_predict(const double *__restrict__ S, long n, float *__restrict__ y,
                                                            const MlpPacked *__restrict__ w) {
   __shared__ __align__(16) MlpPacked M;
@@ -423,8 +455,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS) k_predict(const double *__restr
       Side L, R;
       Gas G;
       SideK kl, kr;
-      load_state(S, n, i, L, R, G, kl, kr);
-      vac = vacuum(L, R, G);
+      vac = load_state(S, n, i, L, R, G, kl, kr) || vacuum(L, R, G);
       if (!vac) features(L, R, G.g, L.p * p_of_w(tr_w(L, R, kl, kr, G), G), f);
     }
     const float yy = mlp_lane(M, f);
@@ -469,8 +500,7 @@ __global__ void k_make_samples(const double *S, const double *out, long n, float
     Side L, R;
     Gas G;
     SideK kl, kr;
-    load_state(S, n, i, L, R, G, kl, kr);
-    if (vacuum(L, R, G)) continue;
+    if (load_state(S, n, i, L, R, G, kl, kr) || vacuum(L, R, G)) continue;
     double ps = out[i];
     if (!(ps > 0.0)) continue;
     double ptr = L.p * p_of_w(tr_w(L, R, kl, kr, G), G);
