@@ -541,8 +541,8 @@ __global__ void __launch_bounds__(TRAIN_THREADS) k_grad(const float *__restrict_
   TrainSmem &s = *reinterpret_cast<TrainSmem *>(smem_raw);
   const int tid = threadIdx.x;
   float *G = part + (size_t)blockIdx.x * PSTRIDE;
-  // the CTA's first tile writes its row, later ones (batches beyond
-  // GRAD_CTAS tiles) add to it
+  // the CTA's first tile writes its row, later ones (batches with more
+  // tiles than CTAs) add to it
   bool first = true;
   auto put = [&](int t, float x) { G[t] = first ? x : G[t] + x; };
   for (int t = tid; t < NH * NIN; t += TRAIN_THREADS) s.W1[t] = w[OFF_W1 + t];
@@ -756,10 +756,10 @@ struct flash_hy_rsolver {
   MlpPacked *packed;            // BF16 inference copy of w
   int *queue, *qcount;          // fallback queue of the learned path
   long qcap;
-  float *part;                  // k_grad's rows [GRAD_CTAS][PSTRIDE]
+  float *part;                  // k_grad's rows [grad_ctas][PSTRIDE], from the first training on
   int *idx;                     // train: the epoch's sample order
   long idx_cap;
-  int grad_set;                 // k_grad's shared-memory limit is raised
+  long grad_ctas;               // CTAs of k_grad at most: two per SM
   unsigned *status;
   int step;
   int infer;                    // FLASH_HY_INFER_TCGEN05 or FLASH_HY_INFER_WARP_MMA
@@ -779,15 +779,21 @@ static int grid_for(long n, int threads) {
   return (int)(g > 0 ? g : 1);
 }
 
-constexpr long GRAD_CTAS = 296;         // two per SM
-static long grad_ctas(long nb) { const long t = (nb + TS - 1) / TS; return t < GRAD_CTAS ? t : GRAD_CTAS; }
+static long grad_ctas(const flash_hy_rsolver *r, long nb) {
+  const long t = (nb + TS - 1) / TS;
+  return t < r->grad_ctas ? t : r->grad_ctas;
+}
 
-// k_grad's shared memory, raised on a solver's first use of it (loading the
-// kernel at create would cost every solver 0.7 ms)
+// what only training needs, on a solver's first use of it: k_grad's shared
+// memory (loading the kernel at create would cost every solver 0.7 ms) and
+// its rows (5.7 MB)
 static int grad_ready(flash_hy_rsolver *r) {
-  if (r->grad_set) return 0;
+  if (r->part) return 0;
+  int sms = 0;
+  RS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, r->device));
   RS_CUDA(cudaFuncSetAttribute(k_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TrainSmem)));
-  r->grad_set = 1;
+  r->grad_ctas = 2L * sms;
+  RS_CUDA(cudaMalloc((void **)&r->part, (size_t)r->grad_ctas * PSTRIDE * sizeof(float)));
   return 0;
 }
 
@@ -834,13 +840,12 @@ extern "C" int flash_hy_rsolver_create(int device, flash_hy_rsolver **out) {
   // one allocation, w at its start
   const size_t row = PSTRIDE * sizeof(float);
   char *mem = nullptr;
-  RS_CUDA(cudaMalloc((void **)&mem, (4 + GRAD_CTAS) * row + 256 + sizeof(MlpPacked)));
+  RS_CUDA(cudaMalloc((void **)&mem, 4 * row + 256 + sizeof(MlpPacked)));
   r->w = (float *)mem;
   r->m = (float *)(mem + row);
   r->v = (float *)(mem + 2 * row);
   r->G = (float *)(mem + 3 * row);
-  r->part = (float *)(mem + 4 * row);
-  mem += (4 + GRAD_CTAS) * row;
+  mem += 4 * row;
   r->packed = (MlpPacked *)mem;
   mem += (sizeof(MlpPacked) + 15) / 16 * 16;
   r->loss = (float *)mem;
@@ -886,7 +891,7 @@ extern "C" int flash_hy_rsolver_destroy(flash_hy_rsolver *r) {
   if (!r) return FLASH_HY_ERR_BAD_ARG;
   cudaSetDevice(r->device);
   if (r->stream) cudaStreamSynchronize(r->stream);
-  cudaFree(r->w); cudaFree(r->queue); cudaFree(r->idx);
+  cudaFree(r->w); cudaFree(r->queue); cudaFree(r->idx); cudaFree(r->part);
   if (r->stream) cudaStreamDestroy(r->stream);
   free(r);
   return 0;
@@ -967,8 +972,8 @@ extern "C" int flash_hy_rsolver_grad(flash_hy_rsolver *r, const float *d_x, cons
   if (!r || !d_x || !d_t || !d_idx || nb <= 0) return FLASH_HY_ERR_BAD_ARG;
   RS_CUDA(cudaSetDevice(r->device));
   if (int e = grad_ready(r)) return e;
-  k_grad<<<(int)grad_ctas(nb), TRAIN_THREADS, sizeof(TrainSmem), r->stream>>>(r->w, d_x, d_t, d_idx, nb, 1.f / nb, r->part);
-  k_reduce<<<RED_GRID, 256, 0, r->stream>>>(r->part, (int)grad_ctas(nb), r->G, r->loss);
+  k_grad<<<(int)grad_ctas(r, nb), TRAIN_THREADS, sizeof(TrainSmem), r->stream>>>(r->w, d_x, d_t, d_idx, nb, 1.f / nb, r->part);
+  k_reduce<<<RED_GRID, 256, 0, r->stream>>>(r->part, (int)grad_ctas(r, nb), r->G, r->loss);
   RS_CUDA(cudaGetLastError());
   if (h_grad) RS_CUDA(cudaMemcpyAsync(h_grad, r->G, NPARAM * sizeof(float), cudaMemcpyDeviceToHost, r->stream));
   if (h_loss) RS_CUDA(cudaMemcpyAsync(h_loss, r->loss, sizeof(float), cudaMemcpyDeviceToHost, r->stream));
@@ -990,7 +995,7 @@ extern "C" int flash_hy_rsolver_train(flash_hy_rsolver *r, const float *d_x, con
     r->idx_cap = ns;
   }
   int *idx = r->idx;
-  const int ctas = (int)grad_ctas(batch);
+  const int ctas = (int)grad_ctas(r, batch);
   float last = 0.f;
   long nbat = ns / batch;
   for (int ep = 0; ep < epochs; ++ep) {

@@ -139,3 +139,20 @@ def test_hydro_out_of_range_matches_oracle(scale, flip):
     h.close()
     for k, l1 in conserved_l1(out, ref, grid).items():
         assert l1 <= 1e-10, (k, l1)
+
+
+@pytest.mark.gpu
+def test_a_solver_holds_no_training_memory():
+    """Creating a solver takes one small allocation (cudaMalloc hands out
+    2 MB); the gradient rows come with the first training."""
+    import torch
+    from flash5_b200.riemann import ExactRiemann
+    first = ExactRiemann(0)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    r = ExactRiemann(0)
+    assert free - torch.cuda.mem_get_info()[0] <= 2 << 20
+    X, T = torch.randn(64, 8, device="cuda:0"), torch.randn(64, device="cuda:0")
+    r.train(X, T, 64, epochs=1, batch=32)
+    r.close()
+    first.close()
