@@ -1195,8 +1195,10 @@ static int enqueue_step(flash_hy_ctx *c, double dt, const int *d_list, int nlaun
   a.sweep = c->p.precision == FLASH_HY_PREC_MIXED && c->mx_sweep == FLASH_HY_SWEEP_ZYX ? 1 : 0;
   a.stream = c->stream;
   a.tma = c->tma_maps ? c->tma_maps + 3 * c->cur : nullptr;
-  // the FP64 kernels give the same bits on runs, so they always take them
-  const bool runs = c->tma_run && (c->mx_runs > 1 || c->p.precision != FLASH_HY_PREC_MIXED);
+  // the FP64 kernels without FMA contraction give the same bits on runs, so
+  // they always take them; the contracted ones (FP64_FMA, mixed) agree to
+  // rounding with their one-block forms and follow the setting
+  const bool runs = c->tma_run && (c->mx_runs > 1 || c->p.precision == FLASH_HY_PREC_FP64);
   a.tma_run = runs ? c->tma_run + 3 * c->cur : nullptr;
   a.nblocks = c->nblocks;
   a.nlev = 0;

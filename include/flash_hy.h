@@ -355,16 +355,18 @@ int flash_hy_mark_refine_tree(flash_hy_ctx *ctx, int nvar, const int *vars, doub
  * trials are dropped; the next flash_hy_compute_dt recomputes dt from the
  * restored state.                                                         */
 #define FLASH_HY_TUNE_MAX 8
-/* mx_runs: blocks a CTA of the mixed-precision 3D direction kernels
- * stages along the sweep -- 1, or FLASH_HY_MX_RUN where the context offers
+/* mx_runs: blocks a CTA of the mixed-precision and FP64_FMA 3D direction
+ * kernels stages along the sweep -- 1, or FLASH_HY_MX_RUN where the context offers
  * runs (a full uniform grid of 8^3 blocks whose block counts divide by it):
  * the CTA then takes runs of FLASH_HY_MX_RUN blocks and a part of their
- * cross-section (a quarter, or an eighth with HLLC, where it has at most
- * 288 threads), which shares the stencil overlap along the sweep.  The FP64
- * direction kernels take the same runs whatever is set: their results are
- * bit-identical either way.  The two are separately compiled FMA-contracted
- * kernels, like the mx_threads candidates, and agree to rounding.  The
- * default is FLASH_HY_MX_RUN where offered; autotune tries both.        */
+ * cross-section (mixed with the exact solver a quarter, else an eighth, with
+ * at most 288 threads), which shares the stencil overlap along the sweep.
+ * The two are separately compiled FMA-contracted kernels, like the
+ * mx_threads candidates, and agree to rounding: a block-list, split or
+ * sharded step, which takes one block per CTA, equals a full step bit for
+ * bit with mx_runs = 1.  The FLASH_HY_PREC_FP64 direction kernels take runs
+ * whatever is set: their results are bit-identical either way.  The default
+ * is FLASH_HY_MX_RUN where offered; autotune tries both on the mixed path. */
 #define FLASH_HY_MX_RUN 4
 /* mx_sweep: the order in which the mixed-precision direction kernels
  * accumulate the conservative update -- FLASH_HY_SWEEP_XYZ (the default)

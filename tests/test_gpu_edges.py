@@ -104,3 +104,33 @@ def test_mixed_vanishing_pressures_close_to_oracle(name):
     h.close()
     for k, l1 in conserved_l1(out, ref, grid).items():
         assert l1 <= 1e-6, (k, l1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rs", [abi.RS_HLLC, abi.RS_EXACT])
+def test_fma_runs_follow_the_setting(rs):
+    """FP64_FMA kernels on runs are compiled (and contracted) apart from the
+    one-block ones: with mx_runs = 1 a full step equals the block-list step
+    bit for bit, on runs to rounding."""
+    grid = UniformGrid(3, (8, 8, 8), (4, 4, 4), bc="periodic")
+    unk = setups.kelvin_helmholtz(grid)
+    params = abi.default_params(gamma=5.0 / 3.0, precision=abi.PREC_FP64_FMA, riemann_solver=rs)
+    out = {}
+    for how in ("runs", "one", "list"):
+        h = Hydro(params, grid)
+        assert h.tuning["mx_runs"] == 4
+        if how == "one":
+            h.tuning = dict(h.tuning, mx_runs=1)
+        h.upload(unk)
+        dt, _ = h.compute_dt()
+        for _ in range(3):
+            if how == "list":
+                h.step_blocks(range(grid.nblocks), 0.0, dt, dt)
+            else:
+                h(0.0, dt, dt)
+        out[how] = grid.new_unk()
+        h.download(out[how])
+        h.close()
+    assert np.array_equal(out["one"], out["list"])
+    # three steps of a state of order one: a few roundings of 1e-16 each
+    assert np.abs(out["runs"] - out["one"])[..., [VAR[v] for v in ("dens", "velx", "vely", "velz", "eint")]].max() <= 1e-13
