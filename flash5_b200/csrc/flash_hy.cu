@@ -1727,7 +1727,10 @@ extern "C" int flash_hy_autotune(flash_hy_ctx *c, double dt, int steps, flash_hy
     float best_ms = 3.4e38f;
     int best_dir = mixed ? sel0 : dir0;
     const int ndir = mixed ? 3 : ncand;
+    // the mixed HLLC kernels on runs have one form: one trial
+    const bool one_form = mixed && c->tma_run && c->mx_runs > 1 && !step_list && c->p.riemann_solver != FLASH_HY_RS_EXACT;
     for (int q = 0; q < ndir && !rc; ++q) {
+      if (one_form && q != sel0) continue;
       if (mixed) c->mx_sel = q; else c->dir_threads = cand[q];
       float ms = 0.f;
       rc = trial(ms);

@@ -54,20 +54,21 @@ static bool launch_dir_one(const StepArgs &a) {
     return false;
   TmaLine tl;
   memset(&tl, 0, sizeof tl);
-  if constexpr (NDIM == 3) {
-    // full uniform grid: runs of kMxRun blocks along the sweep
+  // full uniform grid: runs of kMxRun blocks along the sweep.  An eighth's
+  // phases have at most 288 cells, so the HLLC runs have one form, that of
+  // 288 threads (unit 0, step_mixed); the exact solver's quarters keep the
+  // candidates
+  if constexpr (NDIM == 3 && (RS == 1 || FHY_MXSEL == 0)) {
     if (use_runs(a)) {
       constexpr int Q = run_parts(true, RS == 1);
+      static_assert(Q != 8 || NT == 288, "one pass of every phase of an eighth");
       using GR = MxGeom<NDIM, NX, NY, NZ, DIR, RS, kMxRun, Q>;
-      // an eighth's phases have at most 288 cells; the candidates keep their
-      // own thread counts on quarters
-      constexpr int NTR = Q == 8 && NT > 288 ? 288 : NT;
-      auto kr = k_dir_mx<NDIM, NX, NY, NZ, DIR, FIRST, LAST, RS, NTR, kMxRun, Q, ORD>;
+      auto kr = k_dir_mx<NDIM, NX, NY, NZ, DIR, FIRST, LAST, RS, NT, kMxRun, Q, ORD>;
       const size_t smr = GR::smem_bytes();
       if (a.set_attr && cudaFuncSetAttribute(kr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smr) != cudaSuccess)
         return false;
       tl = a.tma_run[DIR - 1];
-      kr<<<a.nlaunch / kMxRun * Q, NTR, smr, a.stream>>>(a.P, (const Real *)a.sig, a.acc, a.aux, a.ncells, a.part, tl);
+      kr<<<a.nlaunch / kMxRun * Q, NT, smr, a.stream>>>(a.P, (const Real *)a.sig, a.acc, a.aux, a.ncells, a.part, tl);
       if (LAST)
         k_cfl_merge<NX, NY, Q><<<(a.nblocks + 255) / 256, 256, 0, a.stream>>>(a.cflq, nullptr, a.nblocks, a.P.cfl,
                                                                                    a.part);
@@ -224,7 +225,7 @@ int FHY_ENTRY(const StepArgs &a, int ndim, int nx, int ny, int nz) {
 
 #if FHY_VARIANT == 3 && FHY_MXSEL == 0
 int step_mixed(const StepArgs &a, int ndim, int nx, int ny, int nz) {
-  switch (a.mx_sel) {
+  switch (use_runs(a) && a.P.riemann != FLASH_HY_RS_EXACT ? 0 : a.mx_sel) {
     case 0: return step_mixed_nt0(a, ndim, nx, ny, nz);
     case 2: return step_mixed_nt2(a, ndim, nx, ny, nz);
     default: return step_mixed_nt1(a, ndim, nx, ny, nz);

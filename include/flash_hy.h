@@ -340,7 +340,10 @@ int flash_hy_mark_refine_tree(flash_hy_ctx *ctx, int nvar, const int *vars, doub
  * candidates per block shape).  Every face and cell is computed by one
  * thread and the CFL reduction is order independent, so sig_threads and
  * dir_threads leave results bit-identical; the mx_threads candidates are
- * separately compiled FMA-contracted kernels and agree to rounding.
+ * separately compiled FMA-contracted kernels and agree to rounding.  On
+ * runs of blocks (mx_runs) a CTA has at most 288 cells per phase: there the
+ * FP64 kernels launch min(dir_threads, 288) threads, and the mixed HLLC
+ * kernels 288 whatever mx_threads says (one trial of autotune).
  * set_tuning refuses values that are not
  * candidates of the context's block shape (FLASH_HY_ERR_BAD_ARG);
  * tuning_candidates lists them (arrays of FLASH_HY_TUNE_MAX entries).
