@@ -22,7 +22,8 @@
 namespace fhy {
 
 // whether x lies in [lo, 2^300), lo a positive double given by its high word
-__device__ __forceinline__ bool at_least(double x, int lo) { return __double2hiint(x) - lo > 0 && __double2hiint(x) < 0x52B00000; }
+// (negative x have negative high words)
+__device__ __forceinline__ bool at_least(double x, int lo) { return __double2hiint(x) > lo && __double2hiint(x) < 0x52B00000; }
 
 // FP64 HLLC (hy_HLLC.F90:94-311) and the volume flux F_dens / rho of the
 // upwind side; ig = 1/(game - 1), that of the gamma law.  Branch-free: one

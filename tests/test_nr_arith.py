@@ -67,3 +67,42 @@ def test_results_are_one_rounding_off(tmp_path):
         pytest.skip(f"no C compiler: {e}")
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout
+
+
+RANGES = r"""
+#include <math.h>
+#include <stdint.h>
+#include <stdio.h>
+#include <string.h>
+static int hi(double x) { uint64_t u; memcpy(&u, &x, 8); return (int)(uint32_t)(u >> 32); }
+static int in_range(double x) { return (unsigned)hi(x) - 0x2D300000u < 0x25800000u; }
+static int at_least(double x, int lo) { return hi(x) > lo && hi(x) < 0x52B00000; }
+int main(void) {
+  const double v[] = {0., -0., 5e-324, -5e-324, 1e-310, -1e-310, 1e-100, -1e-100, 0x1p-301, 0x1p-300, 1e-16, -1e-16, 1.,
+                      -1., 0x1.fp299, 0x1p300, -0x1p300, 1e308, INFINITY, -INFINITY, NAN, -NAN};
+  const int lo = hi(0x1p-300);
+  for (unsigned k = 0; k < sizeof v / sizeof *v; ++k) {
+    const int in = v[k] >= 0x1p-300 && v[k] < 0x1p300;
+    if (in_range(v[k]) != in) { printf("in_range %g\n", v[k]); return 1; }
+    /* at_least needs the high word above lo's: a double or so above it */
+    if (at_least(v[k], lo) != (in && v[k] >= 0x1.00001p-300)) { printf("at_least %g\n", v[k]); return 1; }
+    if (at_least(v[k], hi(1e-16)) != (in && v[k] > 1.01e-16)) { printf("at_least tiny %g\n", v[k]); return 1; }
+  }
+  return 0;
+}
+"""
+
+
+def test_range_tests(tmp_path):
+    """The tests on high words that choose between the branch-free forms and
+    the general ones (``in_range``, and ``at_least`` of the mixed HLLC), with
+    negative numbers, zeros of both signs, subnormals, infinities and NaN."""
+    c = tmp_path / "ranges.c"
+    exe = tmp_path / "ranges"
+    c.write_text(RANGES)
+    try:
+        subprocess.run(["gcc", "-O2", "-fwrapv", "-o", str(exe), str(c), "-lm"], check=True, capture_output=True, text=True)
+    except (OSError, subprocess.CalledProcessError) as e:
+        pytest.skip(f"no C compiler: {e}")
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout
