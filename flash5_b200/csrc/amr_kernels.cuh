@@ -334,20 +334,18 @@ __device__ __forceinline__ void amr_guard_nb(const DevParams &P, const double *c
 }
 
 // guard cells the step reads: the slabs of four layers on the lines of
-// interior cells, and the cells k_sig stages (the box of one layer and one
-// cell beyond it along one axis)
+// interior cells, and the cells k_sig stages (two layers, SigStage::needed)
 template <int NDIM, int NX, int NY, int NZ>
 __host__ __device__ __forceinline__ bool step_guard(int li, int lj, int lk) {
   const int x[3] = {li, lj, lk}, N[3] = {NX, NY, NZ};
-  int out = 0, beyond = 0;
+  int out = 0;
   bool near = true;
 #pragma unroll
   for (int d = 0; d < NDIM; ++d) {
     out += x[d] < 0 || x[d] >= N[d];
-    beyond += x[d] < -1 || x[d] > N[d];
     near &= x[d] >= -2 && x[d] <= N[d] + 1;
   }
-  return out == 1 || (near && beyond <= 1);
+  return out == 1 || (near && SigStage<NDIM, NX, NY, NZ>::needed(li, lj, lk));
 }
 
 template <int NDIM, int NX, int NY, int NZ>

@@ -674,10 +674,7 @@ extern "C" int flash_hy_create(const flash_hy_params *params, const flash_hy_gri
         c->tma_run = make_tma_maps(c, fhy::run_parts(params->precision == FLASH_HY_PREC_MIXED,
                                                      params->riemann_solver == FLASH_HY_RS_EXACT));
         if (c->tma_run)
-          for (int t = 0; t < 6; ++t) {
-            c->tma_run[t].runs = c->d_runs[t % 3];
-            c->tma_run[t].cflq = c->d_cflq;
-          }
+          for (int t = 0; t < 6; ++t) c->tma_run[t].runs = c->d_runs[t % 3];
         if (c->tma_run) c->mx_runs = K;
       }
     }

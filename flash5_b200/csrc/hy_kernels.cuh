@@ -261,13 +261,12 @@ __device__ __forceinline__ void stage_prims(const DevParams &P, int b, int3 bc, 
   }
 }
 
-// the primitive slots of load_prim<..., GAME> from the staged cell e
-template <bool GAME = false>
+// the primitive slots of load_prim<..., false> from the staged cell e
 __device__ __forceinline__ void staged_prim(const DevParams &P, const double *sQ, int n, int e, double V[8]) {
   const double rho = sQ[e], eg = sQ[4 * n + e];
   const double p = rho * eg * P.gam1inv;
   V[HD] = rho; V[HVX] = sQ[n + e]; V[HVY] = sQ[2 * n + e]; V[HVZ] = sQ[3 * n + e]; V[HP] = p;
-  V[HGC] = P.gamma; V[HGE] = GAME ? p / (eg * rho) + 1 : 0.0; V[HEI] = eg;
+  V[HGC] = P.gamma; V[HGE] = 0.0; V[HEI] = eg;
 }
 
 template <int NDIM, int NX, int NY, int NZ>
@@ -277,7 +276,7 @@ struct SigStage {
   // rho, vx, vy, vz and e (after the guard-cell EOS) of the staged cells; the neighbour table
   static constexpr size_t smem_bytes() { return (size_t)5 * E::n * sizeof(double) + NNB * sizeof(int); }
   // staged: at most one coordinate outside the box [-1, N]
-  __device__ static __forceinline__ bool needed(int i, int j, int k) {
+  __host__ __device__ static __forceinline__ bool needed(int i, int j, int k) {
     const int c[3] = {i, j, k}, n[3] = {NX, NY, NZ};
     int out = 0;
 #pragma unroll

@@ -22,8 +22,8 @@ __host__ __device__ constexpr int run_parts(bool mixed, bool exact) { return mix
 // CFL candidates kept per block, at most (one per CTA that shares it)
 constexpr int kCflParts = 8;
 
-// Tensor maps of the step's input state for the mixed direction kernels'
-// TMA staging (k_dir_mx, uniform 3D grids): per state variable the block
+// Tensor maps of the step's input state for the direction kernels' TMA
+// staging (uniform 3D grids; the FP64 kernels on runs): per state variable the block
 // interior (box 8 x 8 x 8) and the neighbour slab along the sweep direction
 // (box 4 x 8 x 8, 8 x 4 x 8 or 8 x 8 x 4) over the natural block layout;
 // for runs, the same boxes cut to one part of the slower transverse axis.
@@ -32,7 +32,6 @@ struct TmaLine {
   CUtensorMap slab[5];
   int on;                     // 0: the stencil is staged by load_prim
   const int *runs;            // runs: [nblocks / kMxRun][kMxRun + 2] blocks along the sweep, neighbours below / above
-  void *cflq;                 // runs, last direction: [nblocks][parts] CflCand of the parts
 };
 
 struct StepArgs {

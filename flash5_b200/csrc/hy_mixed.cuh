@@ -112,7 +112,7 @@ __device__ __forceinline__ bool hllc_fp64(const DevParams &P, const double *Vm, 
 
 // Lines of a CTA: the block's lines along DIR (K = 1), or, with K > 1, a
 // run of K blocks that follow one another along DIR, of which the CTA takes
-// 1/K of the cross-section (quarter q of the slower transverse axis): the
+// one of Q parts of the cross-section (of its slower transverse axis): the
 // lines are K blocks long, so the stencil overlap along DIR (four guard
 // cells on each side, recomputed slopes and face states at the ends) is
 // paid once per run instead of once per block.
@@ -121,7 +121,7 @@ struct MxGeom {
   static constexpr int ND0 = DIR == 1 ? NX : (DIR == 2 ? NY : NZ);               // block extent along DIR
   static constexpr int ND = K * ND0;                                              // line interior
   static constexpr int T1 = DIR == 1 ? NY : NX;                                   // faster transverse axis
-  static constexpr int T2 = DIR == 3 ? NY : NZ;                                   // slower one (split by K)
+  static constexpr int T2 = DIR == 3 ? NY : NZ;                                   // slower one (split by Q)
   static_assert(Q == 1 || (NDIM == 3 && T2 % Q == 0), "runs split the slower transverse axis");
   static constexpr int T2Q = T2 / Q;
   static constexpr int C = T1 * T2Q;                                              // lines
@@ -155,7 +155,7 @@ struct MxGeom {
     xl = x - m * ND0;
     return m;
   }
-  // block-local cell of block-relative position xl on line l of quarter q
+  // block-local cell of block-relative position xl on line l of part q
   __device__ static __forceinline__ void cell(int xl, int l, int q, int &i, int &j, int &k) {
     const int t1 = l % T1, t2 = l / T1 + q * T2Q;
     if (DIR == 1) { i = xl; j = t1; k = t2; }
@@ -224,7 +224,7 @@ template <int NDIM, int NT, int Q> constexpr int mx_ctas() { return NDIM == 3 ? 
 template <int NDIM, int NX, int NY, int NZ, int DIR, bool FIRST, bool LAST, int RS, int NT, int K = 1, int Q = 1, int ORD = 0>
 __global__ void __launch_bounds__(NT, mx_ctas<NDIM, NT, Q>())
 k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ ACC, double *__restrict__ AUX,
-         size_t ncells, CflPart *part, const __grid_constant__ TmaLine tm) {
+         size_t ncells, CflPart *part, CflCand *cflq, const __grid_constant__ TmaLine tm) {
   static_assert(NT % 32 == 0, "threads per CTA must be a multiple of 32");
   using G = MxGeom<NDIM, NX, NY, NZ, DIR, RS, K, Q>;
   using B = Box<NDIM, NX, NY, NZ>;
@@ -245,9 +245,9 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
   static_assert((6 * B::n * 4) % 16 == 0 && (NCB * 8) % 16 == 0, "bulk prefetch sizes must be multiples of 16 bytes");
   // the tile copies' descriptors load while the block's indices do
   if (NDIM == 3 && tm.on && threadIdx.x < 10) prefetch_tensormap(threadIdx.x < 5 ? &tm.intr[threadIdx.x] : &tm.slab[threadIdx.x - 5]);
-  // the CTA's blocks: one (K = 1), or run blockIdx.x / K of K blocks that
+  // the CTA's blocks: one (K = 1), or run blockIdx.x / Q of K blocks that
   // follow one another along DIR (with the neighbours below and above the
-  // run), of which the CTA takes quarter qtr = blockIdx.x % K
+  // run), of which the CTA takes part qtr = blockIdx.x % Q
   int blk[K], nbs[2] = {-1, -1}, qtr = 0;
   if constexpr (K == 1) {
     blk[0] = P.blk_list ? P.blk_list[blockIdx.x] : blockIdx.x;
@@ -313,13 +313,13 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
     }
     if (threadIdx.x == 0) mbar_init(bar, 1);
     __syncthreads();                          // the barrier is initialised before anyone polls it
-    // copies: the interior of each block of the run (quarter qtr of its
+    // copies: the interior of each block of the run (part qtr of its
     // cross-section) and the slabs of the neighbours along DIR, five
     // variables; one thread issues them (K = 1) or the lanes of warp 0
     // issue one each
     constexpr int NOPS = 5 * (K + 2);
     const int q5[5] = {0, 1, 2, 3, 4};         // staged slots of dens, velx, vely, velz, eint
-    const int qo = qtr * G::T2Q;                 // quarter offset on the slower transverse axis
+    const int qo = qtr * G::T2Q;                 // part offset on the slower transverse axis
     auto copy = [&](int o) {
       const int v = o / (K + 2), r = o % (K + 2);
       double *dst = sV + q5[v] * G::SA;
@@ -987,7 +987,7 @@ k_dir_mx(const DevParams P, const float *__restrict__ SIG, double *__restrict__ 
     } else {
       // (the same max / first-index rule as a reduction over the whole block)
       cfl_parts_reduce<K>(cand, [&](int bm) {
-        return static_cast<CflCand *>(tm.cflq) + (size_t)pick(blk, bm) * Q + qtr;
+        return cflq + (size_t)pick(blk, bm) * Q + qtr;
       });
     }
   }

@@ -68,7 +68,7 @@ static bool launch_dir_one(const StepArgs &a) {
       if (a.set_attr && cudaFuncSetAttribute(kr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smr) != cudaSuccess)
         return false;
       tl = a.tma_run[DIR - 1];
-      kr<<<a.nlaunch / kMxRun * Q, NT, smr, a.stream>>>(a.P, (const Real *)a.sig, a.acc, a.aux, a.ncells, a.part, tl);
+      kr<<<a.nlaunch / kMxRun * Q, NT, smr, a.stream>>>(a.P, (const Real *)a.sig, a.acc, a.aux, a.ncells, a.part, a.cflq, tl);
       if (LAST)
         k_cfl_merge<NX, NY, Q><<<(a.nblocks + 255) / 256, 256, 0, a.stream>>>(a.cflq, nullptr, a.nblocks, a.P.cfl,
                                                                                    a.part);
@@ -76,7 +76,7 @@ static bool launch_dir_one(const StepArgs &a) {
     }
   }
   if (NDIM == 3 && a.tma && a.nlev == 0) tl = a.tma[DIR - 1];
-  kern<<<a.nlaunch, threads, smem, a.stream>>>(a.P, (const Real *)a.sig, a.acc, a.aux, a.ncells, a.part, tl);
+  kern<<<a.nlaunch, threads, smem, a.stream>>>(a.P, (const Real *)a.sig, a.acc, a.aux, a.ncells, a.part, a.cflq, tl);
 #else
   static_assert(ORD == 0, "the FP64 variants sweep x, y, z");
   TmaLine tl;

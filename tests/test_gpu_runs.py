@@ -2,8 +2,8 @@
 
 On a full uniform 3D grid of 8^3 blocks whose block counts divide by 4, the
 mixed-precision direction kernels stage runs of four blocks that follow one
-another along the sweep, a quarter of their cross-section per CTA, and the
-last direction merges the quarters' CFL candidates per block (tuning
+another along the sweep, a part of their cross-section per CTA, and the
+last direction merges the parts' CFL candidates per block (tuning
 mx_runs = 4, the default there); with mx_runs = 1 a CTA takes one block.
 Each cell and face is computed by the same source arithmetic either way,
 but the two are separately compiled FMA-contracted kernels, as the
@@ -76,7 +76,7 @@ def test_runs_match_one_block_per_cta(case):
             assert tuple(l1) == tuple(l2) and abs(d1 - d2) <= 1e-13 * d2, (d1, d2, l1, l2)
             dt_old, dt = dt, next_dt(d1, dt)
         # the run path was the one taken: the step's launches are the dt
-        # store, k_sig, three direction kernels and the quarters' CFL merge
+        # store, k_sig, three direction kernels and the parts' CFL merge
         runs(t + dt, dt, dt_old)
         single(t + dt, dt, dt_old)
         listed.step_blocks(every, t + dt, dt, dt_old)
