@@ -54,17 +54,17 @@ BYTES_PER_ZONE = 80.0          # read + write of 5 FP64 state variables
 # kernels) from ncu captures of the 160^3 KH step (dram__bytes_read.sum +
 # dram__bytes_write.sum over 4.096e6 zones), scaled to the workload by its
 # zone count (traffic grows in proportion)
-TRAFFIC_PER_ZONE = {"fp64": 1250.6, "mixed": 864.4, "mixed_exact": 893.5, "mixed_learned": 893.5}
+TRAFFIC_PER_ZONE = {"fp64": 1523.2, "mixed": 866.2, "mixed_exact": 864.2, "mixed_learned": 864.2}
 # Floating-point operations per zone-update of one step (k_sig + the three
 # direction kernels), counted by ncu on the same 160^3 KH step:
 # smsp__sass_thread_inst_executed_op_{dadd,dmul,dfma,fadd,fmul,ffma}_pred_on
 # (an FMA counts two), divided by the zones; and the FP64 pipe utilisation
 # (sm__pipe_fp64_cycles_active, % of peak over the kernels' active cycles,
 # weighted by their durations).
-FLOPS_PER_ZONE = {"fp64": {"f64": 7626, "f32": 394, "fp64_pipe_pct": 27.1},
-                  "mixed": {"f64": 1192, "f32": 1984, "fp64_pipe_pct": 15.3},
-                  "mixed_exact": {"f64": 2120, "f32": 2035, "fp64_pipe_pct": 19.6},
-                  "mixed_learned": {"f64": 2120, "f32": 2035, "fp64_pipe_pct": 19.6}}
+FLOPS_PER_ZONE = {"fp64": {"f64": 4413, "f32": 35, "fp64_pipe_pct": 39.8},
+                  "mixed": {"f64": 1206, "f32": 1964, "fp64_pipe_pct": 17.1},
+                  "mixed_exact": {"f64": 1793, "f32": 1951, "fp64_pipe_pct": 20.4},
+                  "mixed_learned": {"f64": 1793, "f32": 1951, "fp64_pipe_pct": 20.4}}
 # nominal vector peaks of a B200 at the 1965 MHz maximum SM clock: 148 SMs x
 # 64 FP64 (128 FP32) FMA lanes x 2 flops; no measured FP64/FP32 peak exists
 # for this pool, so the compute fractions are "of nominal"
