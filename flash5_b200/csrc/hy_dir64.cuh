@@ -87,8 +87,11 @@ template <int NDIM> constexpr int dir64_parts() { return NDIM == 3 ? 2 : 1; }
 // Launch bounds (threads, CTAs per SM).  The kernel is bound by dependent
 // FP64 latency, so warps in flight decide: runs hold 27 warps at 72
 // registers with spills to L1 (128^3 step 1.33 ms) against 18 at 96 (1.48)
-// and 16 at 128 (1.9); one-block 3D CTAs 20 warps at 96; 2D 8^2 blocks, one
-// wave of 256^2 zones at 80 registers (step 0.044 ms against 0.054 at 96).
+// and 16 at 128 (1.9); one-block 3D CTAs 20 warps at 96.  2D 8^2 blocks: 24
+// warps at 80 registers, best from 256^2 to 2048^2 zones (step 0.042 / 1.65 ms;
+// 20 warps at 102 registers 0.054 / 1.85, 32 at 64 0.044 / 1.68).  2D 16^2: 20
+// warps at 96 (0.040 / 1.55; 10 warps 0.056 / 2.42; 30 at 64 registers 0.044 /
+// 1.44: better from 1024^2 on, worse below).
 template <int NDIM, int NX, int K> struct Dir64Bounds {
   static constexpr int threads = K > 1 ? 288 : (NDIM == 3 || NX == 16 ? 320 : 128);
   static constexpr int ctas = K > 1 ? 3 : (NDIM == 3 || NX == 16 ? 2 : 6);
@@ -286,7 +289,8 @@ __device__ __forceinline__ void hllc64(const DevParams &P, A &ar, const double *
 // below (96 registers); 1.92 with the bulk L2 prefetch; 1.85 on runs of four
 // blocks; 1.50 with branch-free divisions; 1.33 with three run CTAs per SM
 // and the traced e parked in shared memory.  2D Sod 256^2: 0.090 -> 0.044 ms.
-//   stage    the line stencils (cp.async through the neighbour table)
+//   stage    the line stencils (cp.async through the neighbour table; runs:
+//            TMA tile copies)
 //   slopes   eigensystem, limited slopes and flattening switch of the cells
 //            [-2, N+1] of every line
 //   states   face states W-/W+ of the cells [-1, N]: PPM

@@ -218,7 +218,10 @@ __host__ __device__ constexpr int aux_slot(int d) { return ORD == 0 ? d - 1 : ND
 // cross-section three (27 warps at 72 registers), quarters and one-block 3D
 // CTAs two.  2D: as many as hold 27 warps at 72 registers (a four-quadrant
 // hierarchy's exact-solver step 2.09 ms; two per SM at 96 registers 2.49,
-// four at 56 2.16, one at 116 3.93).
+// four at 56 2.16, one at 116 3.93; uniform grids of 8^2 blocks, 256^2 and
+// 2048^2 zones: exact 0.038 / 1.49 ms against 0.052 / 1.68 at 18 warps and
+// 0.042 / 1.61 at 30, HLLC 0.034 / 1.17 against 0.041 / 1.37 and 0.034 / 1.15;
+// 16^2 blocks: 1.04 HLLC and 1.26 exact at 2048^2 against 1.27 and 1.47 at 18).
 template <int NDIM, int NT, int Q> constexpr int mx_ctas() { return NDIM == 3 ? (Q == 8 ? 3 : 2) : (27 * 32) / NT; }
 
 template <int NDIM, int NX, int NY, int NZ, int DIR, bool FIRST, bool LAST, int RS, int NT, int K = 1, int Q = 1, int ORD = 0>

@@ -201,7 +201,8 @@ class Hydro:
     @property
     def tuning(self):
         """Launch shape of the step (dict): threads per CTA of the step's
-        kernels, blocks per CTA of the mixed 3D direction kernels (mx_runs)
+        kernels, blocks per CTA of the mixed and FP64_FMA 3D direction
+        kernels (mx_runs)
         and the mixed path's sweep order (mx_sweep, abi.SWEEP_XYZ or
         abi.SWEEP_ZYX)."""
         t = abi.Tuning()
