@@ -62,19 +62,16 @@ __device__ __forceinline__ double div_by(double x, double b, double y) {
   return fma(fma(-q, b, x), y, q);
 }
 __device__ __forceinline__ double div_nr(double x, double b) { return div_by(x, b, rcp_nr(b)); }
-// (the product a y in two parts: its rounding would cost half an ulp)
+// (the seeds' low words are zero, so y y is exact; the rounding of a y would
+// cost half an ulp)
 __device__ __forceinline__ double rsqrt_nr(double a) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(a));
-  const double h = a * y, e = fma(-fma(a, y, -h), y, fma(-h, y, 1.0));
+  const double e = fma(-a, __dmul_rn(y, y), 1.0);
   return fma(y * e, fma(e, 0.375, 0.5), y);
 }
 __device__ __forceinline__ double sqrt_nr(double a) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;\n" : "=d"(y) : "d"(a));
-  const double e = fma(-(a * y), y, 1.0);
-  y = fma(y * e, fma(e, 0.375, 0.5), y);
-  const double q = a * y;
+  const double y = rsqrt_nr(a), q = a * y;
   return fma(0.5 * y, fma(-q, q, a), q);
 }
 // whether x > 0 lies in [2^-300, 2^300): operands in that range keep the
@@ -209,8 +206,8 @@ __device__ __forceinline__ void sound(Side &L, Side &R, const Gas &G) {
 // and w and the pressure functions (s from the densities and pressures, not
 // from the sound speeds, whose roundings would add to it).  TEST: behind a
 // branch on fast_pair, which keeps k_solve_tc from spilling (15M learned
-// solves 1.19 ms; without it 1.22; the two-rarefaction kernel is faster
-// without, 4.43 against 4.47 ms for 1e8).
+// solves 1.18 ms, 2.5 % more without it; the two-rarefaction kernel is 1 %
+// faster without).
 template <bool TEST = false>
 __device__ __forceinline__ void setup(Side &L, Side &R, const Gas &G, SideK &kl, SideK &kr) {
   if (TEST && !fast_pair(L, R)) return;

@@ -124,7 +124,7 @@ __device__ __forceinline__ void enqueue(bool pending, long i, int *queue, int *q
 // One instantiation per path, so that the two-rarefaction path does not
 // carry the network's register footprint.  Bound by FP64 issue and latency;
 // 1e8 pairs on B200, two-rarefaction start: 8.84 ms with two powers, IEEE
-// divisions and roots per solve (16 warps per SM) -> 4.43 ms with one power
+// divisions and roots per solve (16 warps per SM) -> 4.28 ms with one power
 // and branch-free arithmetic (exact_rs.cuh) at 64 registers (32 warps).
 // Pairs out of that arithmetic's range follow after the loop, which then
 // holds no call; the learned forms queue them for k_fallback.

@@ -29,10 +29,9 @@ static double rnd(int lo, int hi) { uint64_t m = nx() & 0xFFFFFFFFFFFFFull; int 
 static double cut(double b) { uint64_t u; memcpy(&u, &b, 8); u &= 0xFFFFFFFF00000000ull; memcpy(&b, &u, 8); return b; }
 static double rcp_nr(double b) { const double y = cut(1. / cut(b)), e = fma(-b, y, 1.); return fma(y, fma(e, e, e), y); }
 static double div_by(double x, double b, double y) { const double q = x * y; return fma(fma(-q, b, x), y, q); }
-static double rsqrt_nr(double a) { const double y = cut(1. / sqrt(cut(a))), h = a * y;
-  const double e = fma(-fma(a, y, -h), y, fma(-h, y, 1.)); return fma(y * e, fma(e, .375, .5), y); }
-static double sqrt_nr(double a) { double y = cut(1. / sqrt(cut(a))); const double e = fma(-(a * y), y, 1.);
-  y = fma(y * e, fma(e, .375, .5), y); const double q = a * y; return fma(.5 * y, fma(-q, q, a), q); }
+static double rsqrt_nr(double a) { const double y = cut(1. / sqrt(cut(a))), e = fma(-a, y * y, 1.);
+  return fma(y * e, fma(e, .375, .5), y); }
+static double sqrt_nr(double a) { const double y = rsqrt_nr(a), q = a * y; return fma(.5 * y, fma(-q, q, a), q); }
 static double worst[4]; static long off[4];
 static void take(int k, double got, long double want) {
   int e; frexpl(want, &e);
