@@ -351,7 +351,7 @@ def device_errors(a, b):
 
 
 # ---------------------------------------------------------------------------
-# CPU oracle legs (the checker's C restatement; only these legs run it)
+# CPU oracle legs (the oracle's C restatement; only these legs run it)
 # ---------------------------------------------------------------------------
 def kh_window(nblk, w=8):
     """A window of w^3 blocks of the nblk^3-block KH grid (straddling the
@@ -639,7 +639,8 @@ def amr_run(args, paths, e2e=True, regrid=True, cpu=True, steps=None, warmup=Non
             best, trials = h.autotune(dts[0] if dts is not None else h.compute_dt()[0], steps=2)
             tunings[name] = {"best": best, "trials_ms": {"/".join(str(v) for v in t.values()): round(m, 4)
                                                          for t, m in trials},
-                             "trial_key": "sig_threads/dir_threads/mx_threads/mx_runs/mx_sweep"}
+                             "trial_key": "sig_threads/dir_threads/mx_threads/mx_runs/mx_sweep (on runs FP64 launches "
+                                          "min(dir_threads, 288), mixed HLLC 288 threads)"}
         headline = name == paths[-1]
         sampler = ClockSampler(0) if headline else None
         ms[name], used, launches[name] = run_device(h, steps, warmup, dts=dts, sampler=sampler)
@@ -876,7 +877,8 @@ def main():
             best, trials = hh.autotune(dt0, steps=2)
             tuned = {"best": best, "trials_ms": {"/".join(str(v) for v in t.values()): round(m, 4)
                                                  for t, m in trials},
-                     "trial_key": "sig_threads/dir_threads/mx_threads/mx_runs/mx_sweep"}
+                     "trial_key": "sig_threads/dir_threads/mx_threads/mx_runs/mx_sweep (on runs FP64 launches "
+                                          "min(dir_threads, 288), mixed HLLC 288 threads)"}
         headline = name == paths[-1]
         sampler = ClockSampler(dev) if headline else None
         ms[name], used, launches[name] = run_device(h, args.steps, warmup, dts=dts, sampler=sampler, dist=dist)

@@ -1,7 +1,7 @@
 """ctypes wrapper of the CPU oracle (test infrastructure only).
 
 Only tests/, __graft_entry__.smoke() and bench.py's CPU-baseline leg use
-this module, always as the checker.  The oracle library is built by
+this module, always to check against.  The oracle library is built by
 ``oracle/Makefile`` (``make -C oracle``).
 """
 import ctypes as C
